@@ -36,13 +36,12 @@
 // predecessor drains; kernels of a finished solve return at once. The host
 // reads the state once per replay while the next replay is already queued.
 //
-// Mixed solves on 3x3-block matrices (and FP64 ones with FCU_PERSISTENT=2)
-// run instead as the persistent loop k_pcg_persistent: one cooperative launch
-// per stretch between residual replacements, the tiled SpMV's CTAs resident
-// throughout, two bounded grid barriers per iteration in place of kernel
-// boundaries, and the direction formed from (z, p) pairs where the product
-// reads them. Small scalar systems go to the batched kernel as a single
-// instance (batch.cu).
+// Solves with the point-Jacobi preconditioner run instead as the persistent
+// loop of pcg_loop.cuh whenever the matrix fits it: one cooperative launch per
+// solve, one CTA per SM, bounded grid-wide exchanges in place of kernel
+// boundaries. The kernels above serve block-Jacobi solves, rows too long for
+// the loop, and FCU_PERSISTENT=0. Small scalar systems go to the batched
+// kernel as a single instance (batch.cu).
 
 #include <algorithm>
 #include <atomic>
@@ -50,6 +49,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <string>
+#include <type_traits>
 
 #include "internal.cuh"
 
@@ -246,16 +246,15 @@ __device__ __forceinline__ T bsr3_row(const int* __restrict__ rp, const int* __r
   return s;
 }
 
-// Iterate the rows handled by this warp; emit(node, component, value) once
+// Iterate the rows handled by warp gw of nw; emit(node, component, value) once
 // per output scalar row (from one lane).
 template <int BS, int VPR, bool DIFF, class T, class GX, class Emit>
-__device__ __forceinline__ void spmv_rows(const int* __restrict__ rp, const int* __restrict__ ci,
-                                          const T* __restrict__ val, i64 nrows, const GX& gx, Emit& emit) {
+__device__ __forceinline__ void warp_rows(const int* __restrict__ rp, const int* __restrict__ ci,
+                                          const T* __restrict__ val, i64 nrows, i64 gw, i64 nw, const GX& gx,
+                                          Emit& emit) {
   constexpr int G = (BS == 3) ? 16 : VPR;  // lanes per node row
   const int lane = threadIdx.x & 31;
   const int sub = lane % G;
-  const i64 gw = (blockIdx.x * (i64)blockDim.x + threadIdx.x) >> 5;
-  const i64 nw = ((i64)gridDim.x * blockDim.x) >> 5;
   constexpr int RPW = 32 / G;
   for (i64 base = gw * RPW; base < nrows; base += nw * RPW) {
     const i64 row = base + lane / G;
@@ -268,6 +267,14 @@ __device__ __forceinline__ void spmv_rows(const int* __restrict__ rp, const int*
       if (valid && sub == 0) emit(row, 0, s);
     }
   }
+}
+
+template <int BS, int VPR, bool DIFF, class T, class GX, class Emit>
+__device__ __forceinline__ void spmv_rows(const int* __restrict__ rp, const int* __restrict__ ci,
+                                          const T* __restrict__ val, i64 nrows, const GX& gx, Emit& emit) {
+  const i64 gw = (blockIdx.x * (i64)blockDim.x + threadIdx.x) >> 5;
+  const i64 nw = ((i64)gridDim.x * blockDim.x) >> 5;
+  warp_rows<BS, VPR, DIFF, T>(rp, ci, val, nrows, gw, nw, gx, emit);
 }
 
 // The SpMV's p.Ap: each block stores its sum (fixed order) in the PAP_REGION
@@ -879,373 +886,7 @@ __global__ void __launch_bounds__(VBLOCK, 5) k_update(i64 n, double* __restrict_
   }
 }
 
-// --- persistent PCG (3x3-block tiled operator, point Jacobi) -----------------
-// The iteration loop in one cooperative launch. The CTAs of the tiled SpMV's
-// grid stay resident, and the two grid-wide steps of an iteration (p.Ap
-// before alpha; r.z and r.r before beta and the stopping test) are grid
-// barriers instead of kernel boundaries. Warp 0 keeps streaming the matrix's
-// tiles through the shared-memory ring across iterations (the matrix does not
-// change), so the first tiles of the next product are in flight while the
-// consumer warps update the vectors. No separate direction step: z and p are
-// kept interleaved as pairs zp[i] = (z_i, p_i), the product forms
-// p = z + beta p_old from one pair load per operand, and the update forms the
-// same value for its own elements (same operands, same fused multiply-add)
-// and stores the new pair. Every CTA adds the per-CTA partials in the same
-// fixed order and takes the same decisions on its own copy of the state
-// record; CTA 0 writes that copy back when the loop ends. The loop ends when
-// the solve is over or, in mixed precision, when a residual replacement is due
-// (the host runs it and launches the loop again). Every wait is bounded: a
-// wait that gives up sets the fault flag, and the CTA ends the loop.
-__device__ __forceinline__ float dir_fma(float beta, float pold, float z) { return __fmaf_rn(beta, pold, z); }
-__device__ __forceinline__ double dir_fma(double beta, double pold, double z) { return __fma_rn(beta, pold, z); }
-
-template <class T>
-struct Pair;
-template <>
-struct Pair<float> {
-  using type = float2;
-};
-template <>
-struct Pair<double> {
-  using type = double2;
-};
-
-// The direction operand of the persistent loop. The pairs are written by the
-// same kernel (other CTAs, before the last grid barrier), so they are read
-// with ordinary coherent loads, never through the read-only path.
-template <class T>
-struct XDirPair {
-  using T2 = typename Pair<T>::type;
-  const T2* zp;
-  T beta;
-  __device__ __forceinline__ T operator()(i64 i) const {
-    const T2 v = zp[i];
-    return dir_fma(beta, v.y, v.x);
-  }
-};
-
-// zp[i] = (z[i], p[i]), or with p == nullptr only the z half (after a
-// residual replacement, which recomputes z and keeps p).
-template <class T>
-__global__ void k_zp_pack(const T* __restrict__ z, const T* __restrict__ p, i64 n,
-                          typename Pair<T>::type* __restrict__ zp) {
-  for (i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
-    if (p) zp[i] = {z[i], p[i]};
-    else zp[i].x = z[i];
-  }
-}
-
-constexpr unsigned BARRIER_LIMIT = 1u << 22;  // polls of a grid barrier (~1 us each) before giving up
-
-// Named barrier of the consumer warps (warp 0, the producer, does not join).
-__device__ __forceinline__ void consumer_sync() {
-  asm volatile("bar.sync 1, %0;" ::"r"(32 * SPMV_CONSUMER_WARPS) : "memory");
-}
-
-// Grid barrier, entered by all consumer threads right after a consumer_sync
-// that follows their writes: the first consumer thread of each CTA arrives
-// with a release add (covering its CTA's writes, ordered before it by that
-// CTA barrier), polls the arrival count with relaxed loads until `target`,
-// then an acquire fence; the CTA's consumer warps pass together. False when
-// the poll gave up.
-__device__ __forceinline__ bool grid_barrier(unsigned long long* bar, unsigned long long target, int ctid,
-                                             unsigned limit = BARRIER_LIMIT) {
-  __shared__ int ok_s;
-  if (ctid == 0) {
-    asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(bar) : "memory");
-    int ok = 0;
-    for (unsigned i = 0; i < limit; ++i) {
-      unsigned long long v;
-      asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(bar) : "memory");
-      if (v >= target) {
-        ok = 1;
-        break;
-      }
-      __nanosleep(32);
-    }
-    asm volatile("fence.acq_rel.gpu;" ::: "memory");
-    ok_s = ok;
-  }
-  consumer_sync();
-  return ok_s != 0;
-}
-
-// Sums of the G per-CTA partials src[j * MAXG + 0 .. G) in one fixed order, the same
-// in every CTA: consumer thread t loads partials t, t + NCT, ... (one each
-// while G <= NCT, so the loads are one round trip), each warp adds its lanes
-// in a fixed shuffle tree, and the warps' sums are added in warp order. Called
-// by all consumer threads; the sums are valid in the first consumer thread.
-template <int NV>
-__device__ __forceinline__ void sum_partials(const double* src, int G, int ctid, double (&tot)[NV]) {
-  constexpr int NCT = 32 * SPMV_CONSUMER_WARPS;
-  __shared__ double ws[NV][SPMV_CONSUMER_WARPS];
-  double v[NV];
-#pragma unroll
-  for (int j = 0; j < NV; ++j) {
-    v[j] = 0.0;
-    for (int b = ctid; b < G; b += NCT) v[j] += __ldcg(src + j * MAXG + b);
-    v[j] = warp_sum(v[j]);
-    if ((ctid & 31) == 0) ws[j][ctid >> 5] = v[j];
-  }
-  consumer_sync();
-  if (ctid == 0)
-#pragma unroll
-    for (int j = 0; j < NV; ++j) {
-      double t = 0.0;
-      for (int w = 0; w < SPMV_CONSUMER_WARPS; ++w) t += ws[j][w];
-      tot[j] = t;
-    }
-}
-
-template <bool DIFF, class T, int TR>
-__global__ void __launch_bounds__(SPMV_THREADS, TILED_CTAS_PER_SM) k_pcg_persistent(
-    const int* __restrict__ rp, const int* __restrict__ ci, const T* __restrict__ val, i64 nrows, int cap_blocks,
-    int nstage, i64 n, double* x, double* r, const double* __restrict__ invd, typename Pair<T>::type* zp, T* ap,
-    CgState* st, double* partials, unsigned long long* bar) {
-  using T2 = typename Pair<T>::type;
-  constexpr int BS = 3;
-  constexpr int LPR = 32 * SPMV_CONSUMER_WARPS / TR;
-  constexpr int NCT = 32 * SPMV_CONSUMER_WARPS;  // consumer threads
-  extern __shared__ __align__(128) unsigned char tile_smem[];
-  __shared__ unsigned long long full[MAX_STAGES], empty[MAX_STAGES];
-  __shared__ CgState ls;  // this CTA's copy of the state record
-  __shared__ double red[2][SPMV_CONSUMER_WARPS];
-  __shared__ double alpha_s;
-  __shared__ int stop_s;             // consumers: the loop has ended
-  __shared__ volatile int ended_s;   // consumers -> producer: no more tiles are needed
-  __shared__ volatile int pfault_s;  // producer -> consumers: a ring wait gave up
-  const size_t stage_bytes = tile_stage_bytes<T, TR, BS>(cap_blocks);
-  const i64 ntiles = (nrows + TR - 1) / TR;
-  const i64 G = gridDim.x;
-  const int mytiles = blockIdx.x < ntiles ? (int)((ntiles - blockIdx.x + G - 1) / G) : 0;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (tid == 0) {
-    for (int s = 0; s < nstage; ++s) {
-      mbar_init(&full[s], 1);
-      mbar_init(&empty[s], SPMV_CONSUMER_WARPS);
-    }
-    fence_mbar_init();
-    ended_s = 0;
-    pfault_s = 0;
-  }
-  static_assert(sizeof(CgState) % 4 == 0, "state record copied by words");
-  for (int i = tid; i < (int)(sizeof(CgState) / 4); i += blockDim.x)
-    reinterpret_cast<int*>(&ls)[i] = reinterpret_cast<const int*>(st)[i];
-  __syncthreads();
-
-  if (warp == 0) {
-    // producer: tile q of the stream is tile q % mytiles of the CTA's share
-    if (mytiles == 0 || ls.done || ls.pause) return;
-    int pb0 = 0, pb1 = 0, desc0 = -1;
-    int k = 0;            // tile of the CTA's share
-    int s = 0;            // ring stage
-    unsigned ph = 0;      // phase parity of the stage's current use
-    int issued = 0;       // copies issued, counted up to nstage
-    for (;;) {
-      if ((k & 31) == 0 && desc0 != k) {
-        const i64 t = blockIdx.x + (i64)(k + lane) * G;
-        if (t < ntiles) {
-          pb0 = rp[t * TR];
-          pb1 = rp[min(t * TR + TR, nrows)];
-        }
-        desc0 = k;
-      }
-      int state = 1;  // 1: stage free, 2: loop ended, 3: wait gave up
-      if (lane == 0) {
-        if (issued >= nstage) {
-          state = 3;
-          for (unsigned i = 0; i < WAIT_LIMIT; ++i) {
-            if (mbar_try_wait(&empty[s], ph ^ 1u)) {
-              state = 1;
-              break;
-            }
-            if (ended_s) {
-              state = 2;
-              break;
-            }
-          }
-        } else if (ended_s) {
-          state = 2;
-        }
-      }
-      state = __shfl_sync(FULL, state, 0);
-      if (state != 1) {
-        if (state == 3 && lane == 0) {
-          atomicExch(&st->fault, 1);
-          pfault_s = 1;
-        }
-        break;
-      }
-      const int b0 = __shfl_sync(FULL, pb0, k & 31), b1 = __shfl_sync(FULL, pb1, k & 31);
-      if (lane == 0) {
-        unsigned char* base = tile_smem + s * stage_bytes;
-        TileHeader* h = reinterpret_cast<TileHeader*>(base);
-        unsigned char* rps = base + align128(sizeof(TileHeader));
-        unsigned char* cs = rps + align128((TR + 1) * 4 + 16);
-        unsigned char* vs = cs + align128((size_t)cap_blocks * 4 + 32);
-        const i64 r0 = (blockIdx.x + (i64)k * G) * TR;
-        const int rows = (int)min((i64)TR, nrows - r0);
-        const unsigned rp_bytes = (unsigned)(((rows + 1) * 4 + 15) & ~15);
-        const uintptr_t c_lo = reinterpret_cast<uintptr_t>(ci + b0) & ~(uintptr_t)15;
-        const uintptr_t c_hi = (reinterpret_cast<uintptr_t>(ci + b1) + 15) & ~(uintptr_t)15;
-        const uintptr_t v_lo = reinterpret_cast<uintptr_t>(val + 9 * (i64)b0) & ~(uintptr_t)15;
-        const uintptr_t v_hi = (reinterpret_cast<uintptr_t>(val + 9 * (i64)b1) + 15) & ~(uintptr_t)15;
-        h->b0 = b0;
-        h->rows = rows;
-        h->col_off = (int)(reinterpret_cast<uintptr_t>(ci + b0) - c_lo);
-        h->val_off = (int)(reinterpret_cast<uintptr_t>(val + 9 * (i64)b0) - v_lo);
-        const unsigned cb = (unsigned)(c_hi - c_lo), vb = (unsigned)(v_hi - v_lo);
-        fence_proxy_async();
-        mbar_arrive_expect_tx(&full[s], rp_bytes + cb + vb);
-        bulk_load(rps, rp + r0, rp_bytes, &full[s]);
-        if (cb) bulk_load(cs, reinterpret_cast<const void*>(c_lo), cb, &full[s]);
-        if (vb) bulk_load(vs, reinterpret_cast<const void*>(v_lo), vb, &full[s]);
-      }
-      if (issued < nstage) ++issued;
-      if (++k == mytiles) k = 0;
-      if (++s == nstage) {
-        s = 0;
-        ph ^= 1u;
-      }
-    }
-    // copies still in flight (at most one per stage) land before the CTA exits
-    if (lane == 0)
-      for (int i = 1; i <= issued; ++i) {
-        int s2 = s - i;
-        unsigned p2 = ph;
-        if (s2 < 0) {
-          s2 += nstage;
-          p2 ^= 1u;
-        }
-        mbar_wait(&full[s2], p2);
-      }
-    return;
-  }
-
-  // consumer warps
-  const int ctid = tid - 32;
-  const int sub = lane % LPR;
-  const int row_in_tile = (warp - 1) * (32 / LPR) + lane / LPR;
-  int cs = 0;                  // ring stage of the next tile
-  unsigned cph = 0;            // its phase parity
-  unsigned long long gen = 0;  // grid barriers passed
-  const i64 step = G * NCT;
-  const i64 i0 = (i64)blockIdx.x * NCT + ctid;  // the thread's first vector element
-  bool run = !(ls.done || ls.pause);
-  while (run) {
-    const T beta = (T)ls.beta;
-    // Ap = A p with p = z + beta p_old formed per operand
-    XDirPair<T> gx{zp, beta};
-    EmitApOwn<T, BS> em{ap};
-    bool tiles_ok = true;
-    for (int k = 0; k < mytiles; ++k) {
-      bool got = false;
-      for (unsigned i = 0; i < WAIT_LIMIT; ++i) {
-        if (mbar_try_wait(&full[cs], cph)) {
-          got = true;
-          break;
-        }
-        if (pfault_s) break;
-      }
-      if (!got) {
-        tiles_ok = false;
-        break;
-      }
-      consume_tile<DIFF, T, TR, BS, false>(tile_smem + cs * stage_bytes, cap_blocks, (blockIdx.x + (i64)k * G) * TR,
-                                           row_in_tile, sub, lane, &empty[cs], gx, em);
-      if (++cs == nstage) {
-        cs = 0;
-        cph ^= 1u;
-      }
-    }
-    if (!tiles_ok && lane == 0) atomicExch(&st->fault, 1);
-    double d = warp_sum(em.dot);
-    if (lane == 0) red[0][warp - 1] = d;
-    consumer_sync();
-    if (ctid == 0) {
-      double t = 0.0;
-      for (int w = 0; w < SPMV_CONSUMER_WARPS; ++w) t += red[0][w];
-      partials[PAP_REGION * MAXG + blockIdx.x] = t;
-    }
-    bool ok = grid_barrier(bar, ++gen * (unsigned long long)G, ctid);
-    // alpha from the G partials, added in the same order in every CTA
-    double pap[1] = {0.0};
-    sum_partials<1>(partials + PAP_REGION * MAXG, ok ? (int)G : 0, ctid, pap);
-    if (ctid == 0) {
-      const bool fault = !ok || *reinterpret_cast<volatile int*>(&st->fault) != 0;
-      if (!ok) atomicExch(&st->fault, 1);
-      double a = 0.0;
-      stop_s = alpha_decide(&ls, pap[0], fault, true, &a) ? 0 : 1;
-      alpha_s = a;
-    }
-    consumer_sync();
-    if (stop_s) break;
-    const double alpha = alpha_s;
-    // x += alpha p ; r -= alpha Ap ; z = D^-1 r ; (z, p) stored ; (r.z, r.r)
-    double rz = 0.0, rr = 0.0;
-    // (all loads of an element before its stores: the vectors are not
-    // declared unaliased, so the compiler keeps loads behind earlier stores)
-    for (i64 i = i0; i < n; i += step) {
-      const T2 v = zp[i];
-      const T av = __ldcg(ap + i);
-      const double xv = x[i], rv = r[i], dv = invd[i];
-      const T pi = dir_fma(beta, v.y, v.x);
-      const double ri = rv - alpha * (double)av;
-      const double zi = ri * dv;
-      zp[i] = {(T)zi, pi};
-      x[i] = xv + alpha * (double)pi;
-      r[i] = ri;
-      rz += ri * zi;
-      rr += ri * ri;
-    }
-    rz = warp_sum(rz);
-    rr = warp_sum(rr);
-    if (lane == 0) {
-      red[0][warp - 1] = rz;
-      red[1][warp - 1] = rr;
-    }
-    consumer_sync();
-    if (ctid == 0) {
-      double a = 0.0, b = 0.0;
-      for (int w = 0; w < SPMV_CONSUMER_WARPS; ++w) {
-        a += red[0][w];
-        b += red[1][w];
-      }
-      partials[blockIdx.x] = a;
-      partials[MAXG + blockIdx.x] = b;
-    }
-    ok = grid_barrier(bar, ++gen * (unsigned long long)G, ctid);
-    double sums[2] = {0.0, 0.0};
-    sum_partials<2>(partials, ok ? (int)G : 0, ctid, sums);
-    if (ctid == 0) {
-      if (!ok || *reinterpret_cast<volatile int*>(&st->fault) != 0) {
-        if (!ok) atomicExch(&st->fault, 1);
-        ls.done = 1;
-        ls.status = FCU_ERR_CUDA;
-      } else if (sizeof(T) == 8) {
-        decide_after_update(&ls, sums[0], sums[1]);
-      } else {
-        decide_after_update_mixed(&ls, sums[0], sums[1]);
-      }
-      stop_s = (ls.done || ls.pause) ? 1 : 0;
-    }
-    consumer_sync();
-    run = stop_s == 0;
-  }
-  if (ctid == 0) {
-    ended_s = 1;
-    if (blockIdx.x == 0) {
-      st->rz = ls.rz;
-      st->beta = ls.beta;
-      st->rr = ls.rr;
-      st->iter = ls.iter;
-      st->done = ls.done;
-      st->status = ls.status;
-      st->do_update = ls.do_update;
-      st->pause = ls.pause;
-    }
-  }
-}
+#include "pcg_loop.cuh"
 
 // Block-Jacobi variant (FP64). Tiles of 96 block rows (288 dofs, one thread
 // per dof): x, r, p, Ap and the thread's row of the inverse block are read
@@ -1604,6 +1245,19 @@ void build_row_blocks(fcu_ctx ctx, const int* rp_dev, i64 nrows, DBuf<int>& rb, 
 // Workspace and host driver
 // ---------------------------------------------------------------------------
 
+// How the persistent loop cuts a matrix into tiles (loop_plan).
+struct LoopPlan {
+  int state = 0;     // 0 not made yet, 1 fits, -1 does not fit
+  int lpr = 0;       // lanes per row
+  int tr = 0;        // most rows of a tile
+  i64 ntiles = 0;
+  DBuf<int> tb;      // tile row bounds, or empty: tr rows each
+  bool pair = false;  // (z, p) pairs and two exchanges per iteration
+  int nstage = 0;
+  int resident = 0;
+  unsigned off_c = 0, off_v = 0, stage = 0;
+};
+
 struct Workspace {
   fcu_ctx ctx = nullptr;
   i64 n = 0;
@@ -1611,9 +1265,10 @@ struct Workspace {
   DBuf<double> z64, pa64, pb64, ap64;  // FP64 path: z, p (two buffers), Ap
   DBuf<float> z32, pa32, pb32, ap32;   // mixed path
   DBuf<CgState> st;
-  DBuf<unsigned long long> bar;  // arrival count of the persistent loop's grid barriers
-  DBuf<float2> zp32;             // persistent loop: (z, p) pairs, mixed
-  DBuf<double2> zp64;            // persistent loop: (z, p) pairs, FP64
+  DBuf<ExchangeMem> ex;  // exchanges of the persistent loop
+  DBuf<float2> zp32;    // its (z, p) pairs, mixed
+  DBuf<double2> zp64;   // and FP64
+  LoopPlan plan[2];     // persistent loop: tiles and ring (FP64, FP32)
   CgState* host_st = nullptr;  // two pinned records: [0] set-up and final state, [0]/[1] alternate between replays
   cudaEvent_t ev[2] = {nullptr, nullptr};  // a replay's state record has arrived on the host
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
@@ -1740,10 +1395,6 @@ Workspace* ensure_ws(fcu_matrix m, bool mixed) {
     for (auto& e : w->ev) CUDA_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     w->vpr = pick_vpr(m);
     w->vpr32 = w->vpr;
-    if (m->bs == 1 && use_stream_spmv(m)) {
-      ensure_row_blocks(m);
-      w->stream[0] = w->stream[1] = true;
-    }
     w->grid = solver_grid(ctx, n);
     // one wave of the update kernel (its first two elements per thread are
     // fetched before the dependency wait, which only resident blocks do early)
@@ -2043,52 +1694,164 @@ void enqueue_iteration(fcu_matrix m, Workspace* w, bool mixed, int parity) {
 
 int launches_per_iteration() { return fuse_direction() ? 2 : 3; }
 
-// The persistent loop (k_pcg_persistent) runs on 3x3-block matrices on the
-// tiled SpMV with point-Jacobi preconditioning.
-bool persistent_capable(fcu_matrix m) {
-  return m->bs == 3 && use_tiled_spmv() && !m->bdinv.p && !fuse_direction();
+// Longest row of the node pattern, 0 where it is not known.
+int known_max_row(fcu_matrix m) { return m->space ? m->space->max_row : m->max_row_own; }
+
+// Byte layout of a stage for tiles of at most `tr` rows and `cap` entries.
+void stage_layout(LoopPlan& P, int bs, size_t wv, int tr, i64 cap) {
+  const size_t rp = align128(sizeof(TileHeader));
+  const size_t c = rp + align128((size_t)(tr + 1 + 3) * 4 + 16);
+  const size_t v = c + align128((size_t)cap * 4 + 32);
+  P.off_c = (unsigned)c;
+  P.off_v = (unsigned)v;
+  P.stage = (unsigned)(v + align128((size_t)cap * bs * bs * wv + 32));
 }
 
-// Which solves take the persistent loop: mixed precision by default (on B200
-// at 421k and 1.57M elasticity dofs it beats the per-iteration graph by
-// 3-6% per iteration); FP64 keeps the graph, whose tiled SpMV gathers one
-// 8-byte operand per component instead of the loop's 16-byte (z, p) pair
-// (equal at 421k dofs, 12% faster at 1.57M). FCU_PERSISTENT=0 keeps the graph
-// for both, FCU_PERSISTENT=2 takes the loop for both.
-bool use_persistent(fcu_matrix m, bool mixed) {
+// Lanes per scalar row of the persistent loop: as many as leave a lane about
+// eight entries, the number whose operands it fetches in one go.
+int loop_lanes(double mean) { return mean <= 8.0 ? 1 : mean <= 16.0 ? 2 : mean <= 32.0 ? 4 : 8; }
+
+// Matrices of at most this many bytes take the form of the loop with (z, p)
+// pairs and two exchanges per iteration, larger ones the form with a plain
+// direction and three: about what the SMs' shared memory holds. Below it an
+// exchange costs more than the pairs' wider gathers, above it less. Measured
+// (us per iteration, pairs against plain): FP64 12 MB 9.1 / 10.7, 20 MB
+// 11.2 / 11.5, 41 MB 17.9 / 18.1, 46 MB 16.1 / 15.2, 154 MB 43.2 / 36.0; mixed
+// 11 MB 9.6 / 10.8, 24 MB 12.2 / 13.3, 33 MB 17.7 / 19.0, 61 MB 22.6 / 22.4,
+// 81 MB 27.7 / 26.4.
+constexpr double PAIR_BYTES = 36e6;
+
+// Tiles and ring of the persistent loop for m, made once per matrix and
+// precision; nullptr when the matrix does not fit it (no rows, or rows so
+// long that three tiles of one row exceed shared memory).
+//  - A tile holds at most the rows the consumer warps take at once, fewer
+//    where the rows are long: three stages have to fit.
+//  - Where the rows are of about equal length (longest <= 1.25 x mean, and
+//    for 3x3 blocks always) tiles are equal row ranges, evened out over the
+//    CTAs. Elsewhere (P2: vertex rows are twice as long as edge rows) equal
+//    ranges would leave half of each stage empty, so the bounds are cut on
+//    the host to an entry budget of a quarter of shared memory.
+LoopPlan* loop_plan(fcu_matrix m, Workspace* w, bool mixed) {
+  LoopPlan& P = w->plan[mixed ? 1 : 0];
+  if (P.state) return P.state > 0 ? &P : nullptr;
+  P.state = -1;
+  fcu_ctx ctx = m->ctx;
+  const i64 nr = m->nnodes;
+  if (nr <= 0 || m->nnzb <= 0 || ctx->num_sms > EX_MAX_CTAS || m->n > 2000000000) return nullptr;
+  int optin = 0;
+  CUDA_CHECK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+  const size_t budget = (size_t)optin - 2048;  // the kernel's static arrays
+  const size_t wv = mixed ? 4 : 8;
+  const int bs = m->bs, G = ctx->num_sms;
+  const double mean = (double)m->nnzb / (double)nr;
+  P.pair = (double)m->nnzb * (4.0 + (double)wv * bs * bs) <= PAIR_BYTES;
+  P.lpr = bs == 1 ? loop_lanes(mean) : mixed ? LoopShape<3, true, float>::LPR3 : LoopShape<3, true, double>::LPR3;
+  // rows the consumer warps take at once, an even number
+  auto at_once = [&](auto shape) { return (32 * decltype(shape)::W / P.lpr * decltype(shape)::R) & ~1; };
+  auto rows = [&](auto pair) {
+    constexpr bool PR = decltype(pair)::value;
+    if (bs == 3) return mixed ? at_once(LoopShape<3, PR, float>()) : at_once(LoopShape<3, PR, double>());
+    return mixed ? at_once(LoopShape<1, PR, float>()) : at_once(LoopShape<1, PR, double>());
+  };
+  const int trmax = P.pair ? rows(std::true_type()) : rows(std::false_type());
+  const int mr = known_max_row(m);
+  if (mr > 0 && (bs == 3 || mr <= 1.25 * mean)) {
+    int tr = trmax;
+    for (; tr > 0; tr = tr > 8 ? tr - 2 : tr - 1) {
+      stage_layout(P, bs, wv, tr, (i64)tr * mr);
+      if (3 * (size_t)P.stage <= budget) break;
+    }
+    if (tr <= 0) return nullptr;
+    const i64 waves = (nr + (i64)G * tr - 1) / ((i64)G * tr);
+    P.tr = (int)std::min<i64>(tr, (nr + G * waves - 1) / (G * waves));
+    if (P.tr & 1 && P.tr < tr) ++P.tr;
+    stage_layout(P, bs, wv, P.tr, (i64)P.tr * mr);
+    P.ntiles = (nr + P.tr - 1) / P.tr;
+    if (P.tr & 1) P.pair = false;
+  } else {
+    P.pair = false;
+    P.tr = (int)std::min<i64>(trmax, (nr + G - 1) / G);
+    stage_layout(P, bs, wv, P.tr, 0);
+    const size_t per = 4 + wv * bs * bs;
+    const i64 cap = ((i64)budget / 4 - (i64)P.stage - 256) / (i64)per;
+    if (cap <= 0) return nullptr;
+    std::vector<int> rp(nr + 1);
+    CUDA_CHECK(cudaMemcpyAsync(rp.data(), m->row_ptr, (nr + 1) * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
+    std::vector<int> tb;
+    tb.push_back(0);
+    i64 most = 0;
+    for (i64 r = 0; r < nr;) {
+      if (rp[r + 1] - rp[r] > cap) return nullptr;  // a row longer than a tile holds
+      i64 e = r;
+      while (e < nr && e - r < P.tr && (i64)rp[e + 1] - rp[r] <= cap) ++e;
+      most = std::max<i64>(most, rp[e] - rp[r]);
+      tb.push_back((int)e);
+      r = e;
+    }
+    P.ntiles = (i64)tb.size() - 1;
+    upload(ctx, P.tb, tb.data(), tb.size());
+    CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
+    stage_layout(P, bs, wv, P.tr, most);
+  }
+  const i64 waves = (P.ntiles + G - 1) / G;
+  P.nstage = (int)std::min<i64>(MAX_RING, (i64)(budget / P.stage));
+  P.resident = waves <= P.nstage ? 1 : 0;
+  if (P.resident) P.nstage = (int)waves;
+  P.state = 1;
+  return &P;
+}
+
+// Which solves take the persistent loop: those with a point-Jacobi
+// preconditioner whose matrix fits it. FCU_PERSISTENT=0 keeps the
+// per-iteration graph for all.
+LoopPlan* use_persistent(fcu_matrix m, Workspace* w, bool mixed) {
   static int v = [] {
     const char* e = getenv("FCU_PERSISTENT");
     return e ? atoi(e) : 1;
   }();
-  return persistent_capable(m) && (v == 2 || (v == 1 && mixed));
+  if (!v || m->bdinv.p || !use_tiled_spmv()) return nullptr;
+  return loop_plan(m, w, mixed);
 }
 
-// One cooperative launch of the persistent loop: the tiled SpMV's ring and
-// CTAs (up to TILED_CTAS_PER_SM per SM, all resident); the launch fails
-// rather than run when they cannot all be resident. The caller zeroes the
-// barrier count (w->bar) on the stream first.
-template <bool DIFF, class T, int TR>
-void launch_persistent_tr(fcu_matrix m, Workspace* w, const T* val, typename Pair<T>::type* zp, T* ap) {
+// One cooperative launch of the persistent loop, one CTA per SM (the launch
+// fails rather than run when they cannot all be resident), after zeroing
+// its exchange memory.
+template <int BS, int LPR, bool DIFF, bool PAIR, class T>
+void launch_loop(fcu_matrix m, Workspace* w, const LoopPlan& P, const T* val, T* p, typename Pair<T>::type* zp, T* ap) {
   fcu_ctx ctx = m->ctx;
-  const int cap = TR * max_block_row(m);
-  const size_t stage = tile_stage_bytes<T, TR, 3>(cap);
-  const int nstage = fitted_stages(ctx, w->stages[sizeof(T) == 4 ? 1 : 0], stage);
-  const size_t smem = nstage * stage;
-  auto kern = k_pcg_persistent<DIFF, T, TR>;
-  static int configured_dev = -1;
-  static size_t configured_smem = 0;
-  if (configured_dev != ctx->device || configured_smem < smem) {
-    CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured_dev = ctx->device;
-    configured_smem = smem;
-  }
-  int per_sm = 0;
-  CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, SPMV_THREADS, smem));
-  if (per_sm < 1) fail(FCU_ERR_UNSUPPORTED, "rows too long for the tiled SpMV");
-  const int grid = std::min(MAXG, std::min(per_sm, TILED_CTAS_PER_SM) * ctx->num_sms);
+  if (!w->ex.p) w->ex.alloc(1);
+  CUDA_CHECK(cudaMemsetAsync(w->ex.p, 0, sizeof(ExchangeMem), ctx->stream));
+  LoopArgs<T> a;
+  a.rp = m->row_ptr;
+  a.ci = m->col_idx;
+  a.val = val;
+  a.tb = P.tb.p;
+  a.nrows = m->nnodes;
+  a.ntiles = P.ntiles;
+  a.n = m->n;
+  a.tr = P.tr;
+  a.nstage = P.nstage;
+  a.resident = P.resident;
+  a.off_c = P.off_c;
+  a.off_v = P.off_v;
+  a.stage = P.stage;
+  a.val64 = m->val64.p;
+  a.b = w->b.p;
+  a.x = w->x.p;
+  a.r = w->r.p;
+  a.invd = w->invd.p;
+  a.p = p;
+  a.zp = zp;
+  a.ap = ap;
+  a.st = w->st.p;
+  a.ex = w->ex.p;
+  auto kern = k_pcg_loop<BS, LPR, DIFF, PAIR, T>;
+  const size_t smem = (size_t)P.nstage * P.stage;
+  CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(SPMV_THREADS);
+  cfg.gridDim = dim3(ctx->num_sms);
+  cfg.blockDim = dim3(32 * (LoopShape<BS, PAIR, T>::W + 1));
   cfg.dynamicSmemBytes = smem;
   cfg.stream = ctx->stream;
   cudaLaunchAttribute attr[1];
@@ -2096,62 +1859,49 @@ void launch_persistent_tr(fcu_matrix m, Workspace* w, const T* val, typename Pai
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, m->row_ptr, m->col_idx, val, m->nnodes, cap, nstage, m->n, w->x.p,
-                                w->r.p, (const double*)w->invd.p, zp, ap, w->st.p, w->partials.p, w->bar.p));
+  CUDA_CHECK(cudaLaunchKernelEx(&cfg, kern, a));
   ctx->launches++;
 }
 
-// The (z, p) pairs of the persistent loop from the solver's z and p vectors;
-// with_p false refreshes only the z half (after a residual replacement).
-void pack_zp(fcu_matrix m, Workspace* w, bool mixed, bool with_p) {
-  fcu_ctx ctx = m->ctx;
-  const i64 n = m->n;
-  const int g = grid_for(n, 256, ctx->num_sms * 8);
-  if (mixed) {
-    if (!w->zp32.p) w->zp32.alloc(n);
-    k_zp_pack<float><<<g, 256, 0, ctx->stream>>>(w->z32.p, with_p ? w->pa32.p : nullptr, n, w->zp32.p);
-  } else {
-    if (!w->zp64.p) w->zp64.alloc(n);
-    k_zp_pack<double><<<g, 256, 0, ctx->stream>>>(w->z64.p, with_p ? w->pa64.p : nullptr, n, w->zp64.p);
-  }
-  LAUNCH_CHECK(ctx);
+template <int BS, int LPR4, int LPR8, bool PAIR>
+void launch_loop_prec(fcu_matrix m, Workspace* w, const LoopPlan& P, bool mixed) {
+  if (mixed) launch_loop<BS, LPR4, true, PAIR, float>(m, w, P, m->val32.p, w->pa32.p, w->zp32.p, w->ap32.p);
+  else launch_loop<BS, LPR8, false, PAIR, double>(m, w, P, m->val64.p, w->pa64.p, w->zp64.p, w->ap64.p);
 }
 
-// One launch of the persistent loop in the solve's precision, after zeroing
-// its barrier count.
-void launch_persistent(fcu_matrix m, Workspace* w, bool mixed) {
-  fcu_ctx ctx = m->ctx;
-  if (!w->bar.p) w->bar.alloc(1);
-  CUDA_CHECK(cudaMemsetAsync(w->bar.p, 0, sizeof(unsigned long long), ctx->stream));
-  if (mixed) {
-    if (tile_rows(4) == 64) launch_persistent_tr<true, float, 64>(m, w, m->val32.p, w->zp32.p, w->ap32.p);
-    else launch_persistent_tr<true, float, 32>(m, w, m->val32.p, w->zp32.p, w->ap32.p);
-  } else {
-    launch_persistent_tr<false, double, 32>(m, w, m->val64.p, w->zp64.p, w->ap64.p);
+void launch_persistent(fcu_matrix m, Workspace* w, const LoopPlan& P, bool mixed) {
+  if (P.pair && mixed && !w->zp32.p) w->zp32.alloc(m->n);
+  if (P.pair && !mixed && !w->zp64.p) w->zp64.alloc(m->n);
+  if (m->bs == 3) {
+    constexpr int L4 = LoopShape<3, true, float>::LPR3, L8 = LoopShape<3, true, double>::LPR3;
+    if (P.pair) launch_loop_prec<3, L4, L8, true>(m, w, P, mixed);
+    else launch_loop_prec<3, L4, L8, false>(m, w, P, mixed);
+    return;
   }
+#define FCU_LOOP_CASE(L)                                           \
+  case L:                                                          \
+    if (P.pair) launch_loop_prec<1, L, L, true>(m, w, P, mixed);   \
+    else launch_loop_prec<1, L, L, false>(m, w, P, mixed);         \
+    break;
+  switch (P.lpr) {
+    FCU_LOOP_CASE(1)
+    FCU_LOOP_CASE(2)
+    FCU_LOOP_CASE(4)
+    FCU_LOOP_CASE(8)
+    default: fail(FCU_ERR_UNSUPPORTED, "lanes per row of the persistent loop");
+  }
+#undef FCU_LOOP_CASE
 }
 
-// Runs the solve to its end through the persistent loop: one launch in FP64;
-// in mixed precision one per stretch between residual replacements, each
-// replacement run by k_mx_replace between them.
-void run_persistent(fcu_matrix m, Workspace* w, bool mixed, i64 max_iter) {
+// Runs the solve to its end through the persistent loop, in one launch.
+void run_persistent(fcu_matrix m, Workspace* w, const LoopPlan& P, bool mixed) {
   fcu_ctx ctx = m->ctx;
   CgState* hs = w->host_st;
-  pack_zp(m, w, mixed, true);
-  for (i64 round = 0; round <= max_iter + 1; ++round) {
-    launch_persistent(m, w, mixed);
-    CUDA_CHECK(cudaMemcpyAsync(hs, w->st.p, sizeof(CgState), cudaMemcpyDeviceToHost, ctx->stream));
-    CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
-    if (hs->done || hs->fault || !(mixed && hs->pause)) break;
-    // r = b - A64 x, z = D^-1 r, and the state's replacement step
-    DISPATCH_ROWS(m->bs, w->vpr, w->grid, K_REPLACE, m->row_ptr, m->col_idx, m->val64.p, m->nnodes, w->x.p, w->b.p,
-                  w->invd.p, w->r.p, w->z32.p, w->st.p, w->partials.p);
-    pack_zp(m, w, mixed, false);
-  }
-  if (hs->fault && !hs->done) {
+  launch_persistent(m, w, P, mixed);
+  CUDA_CHECK(cudaMemcpyAsync(hs, w->st.p, sizeof(CgState), cudaMemcpyDeviceToHost, ctx->stream));
+  CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
+  if (hs->fault) {
     hs->done = 1;
-    hs->status = FCU_ERR_CUDA;
-  } else if (hs->fault) {
     hs->status = FCU_ERR_CUDA;
   }
 }
@@ -2292,7 +2042,8 @@ int run_pcg(fcu_matrix m, const double* b_dev, const double* x0_dev, double* x_d
     ensure_inv_diag(m, w);
   }
   if (mixed) build_rowsum32(m);
-  tune_spmv(m, w, mixed);  // first solve in this precision only
+  LoopPlan* plan = use_persistent(m, w, mixed);
+  if (!plan) tune_spmv(m, w, mixed);  // first solve in this precision only
 
   CgState init{};
   init.tol = tol;
@@ -2313,17 +2064,26 @@ int run_pcg(fcu_matrix m, const double* b_dev, const double* x0_dev, double* x_d
                   w->r.p, w->z64.p, w->pa64.p, n, w->st.p, w->partials.p);
   if (!mixed && m->bdinv.p)
     launch_pdl(ctx, k_block_init, w->vgrid, m->nnodes, w->r.p, m->bdinv.p, w->z64.p, w->st.p, w->partials.p);
-  CUDA_CHECK(cudaMemcpyAsync(w->host_st, w->st.p, sizeof(CgState), cudaMemcpyDeviceToHost, ctx->stream));
-  CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
+  // The loop reads the state itself; only the zero right-hand side of the GPU
+  // solvers' rules has to be known here first.
+  const bool direct = plan && max_iter > 0 && !gpu_semantics;
+  if (direct) {
+    run_persistent(m, w, *plan, mixed);
+  } else {
+    CUDA_CHECK(cudaMemcpyAsync(w->host_st, w->st.p, sizeof(CgState), cudaMemcpyDeviceToHost, ctx->stream));
+    CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
+  }
   bool zero_rhs = gpu_semantics && w->host_st->bnorm == 0.0;
-  if (zero_rhs) {
+  if (direct) {
+    // done
+  } else if (zero_rhs) {
     // gpu.rs:1169-1180: zero right-hand side -> zero solution, Ok
     CUDA_CHECK(cudaMemsetAsync(x_dev, 0, n * sizeof(double), ctx->stream));
     w->host_st->done = 1;
     w->host_st->status = FCU_OK;
     w->host_st->iter = 0;
-  } else if (!w->host_st->done && max_iter > 0 && use_persistent(m, mixed)) {
-    run_persistent(m, w, mixed, max_iter);
+  } else if (!w->host_st->done && max_iter > 0 && plan) {
+    run_persistent(m, w, *plan, mixed);
   } else if (!w->host_st->done && max_iter > 0) {
     // Replays of CHUNK iterations, each followed by a copy of the state
     // record to the host. The host keeps one replay queued beyond the one
@@ -2502,6 +2262,10 @@ void tune_spmv(fcu_matrix m, Workspace* w, bool mixed) {
   const int k = mixed ? 1 : 0;
   if (w->tuned[k]) return;
   w->tuned[k] = true;
+  if (m->bs == 1 && use_stream_spmv(m)) {
+    ensure_row_blocks(m);
+    w->stream[k] = true;
+  }
   if (!tuning_enabled()) return;
   fcu_ctx ctx = m->ctx;
   const std::array<i64, 5> key = {m->bs, m->n, m->nnzb, max_block_row(m), k};
@@ -2676,10 +2440,10 @@ void time_spmv_cold_impl(fcu_matrix m, int precision, int reps, size_t flush_byt
   *bytes = (double)m->nnzb * (bs2 * wv + 4.0) + 4.0 * (double)(m->nnodes + 1) + 2.0 * (double)m->n * wv;
 }
 
-// Algorithmic bytes of one iteration of the persistent loop: the matrix
-// (values, columns, row pointers) once; the product reads z and p_old and
-// writes Ap; the update reads x, r, D^-1 (8-byte) and p_old, z, Ap, and
-// writes x, r (8-byte) and p, z.
+// Algorithmic bytes of one iteration of the persistent loop with (z, p) pairs:
+// the matrix (values, columns, row pointers) once; the product reads z and
+// p_old and writes Ap; the update reads x, r, D^-1 (8-byte) and p_old, z, Ap,
+// and writes x, r (8-byte) and p, z. (The plain form moves the same within 10%.)
 double persistent_bytes_per_iter(fcu_matrix m, bool mixed) {
   const double w = mixed ? 4.0 : 8.0;
   const double n = (double)m->n;
@@ -2693,27 +2457,37 @@ double persistent_bytes_per_iter(fcu_matrix m, bool mixed) {
 // the mean over `reps` launches, each from a fresh start.
 // Self-check of the bounded waits the persistent loop and the tiled SpMV
 // rely on, with `limit` polls each. One CTA of the tiled kernels' shape:
-// its consumer threads wait at a grid barrier whose count can never be
-// reached (target 2 with one CTA arriving) and then at the same target,
-// which their second arrival reaches; warp 0 waits on an mbarrier nothing arrives at and then
-// on one whose single arrival it makes. out = {first grid wait passed,
-// second grid wait passed, first mbarrier wait passed, second mbarrier wait
+// its consumer threads wait for an exchange with a second CTA that does not
+// exist and then for one among themselves alone; warp 0 waits on an mbarrier
+// nothing arrives at and then on one whose single arrival it makes. out = {first exchange passed,
+// second exchange passed, first mbarrier wait passed, second mbarrier wait
 // passed}; a correct build gives {0, 1, 0, 1}.
-__global__ void __launch_bounds__(SPMV_THREADS) k_wait_limits(unsigned long long* bar, unsigned limit,
+__global__ void __launch_bounds__(SPMV_THREADS) k_wait_limits(ExchangeMem* mem, unsigned limit,
                                                               int* __restrict__ out) {
   __shared__ unsigned long long mb[2];
+  __shared__ int bad, failed;
   const int tid = threadIdx.x;
   if (tid == 0) {
     mbar_init(&mb[0], 1);
     mbar_init(&mb[1], 1);
     fence_mbar_init();
+    bad = failed = 0;
   }
   __syncthreads();
   if (tid >= 32) {
-    const int ctid = tid - 32;
-    const bool a = grid_barrier(bar, 2, ctid, limit);
-    const bool b = grid_barrier(bar, 2, ctid, limit);  // the count is now 2
-    if (ctid == 0) {
+    constexpr int W = SPMV_CONSUMER_WARPS;
+    Exchange<W> ex;
+    ex.mem = mem;
+    ex.ctid = tid - 32;
+    ex.G = 2;  // the second CTA does not exist
+    ex.post_arrival(&failed);
+    const bool a = ex.wait_arrivals(&bad, limit);
+    consumer_sync<W>();
+    if (ex.ctid == 0) bad = 0;
+    ex.G = 1;  // two exchanges, two arrivals
+    ex.post_arrival(&failed);
+    const bool b = ex.wait_arrivals(&bad, limit);
+    if (ex.ctid == 0) {
       out[0] = a ? 1 : 0;
       out[1] = b ? 1 : 0;
     }
@@ -2725,13 +2499,13 @@ __global__ void __launch_bounds__(SPMV_THREADS) k_wait_limits(unsigned long long
 }
 
 void check_wait_limits_impl(fcu_ctx ctx, unsigned limit, int* results_host) {
-  DBuf<unsigned long long> bar;
+  DBuf<ExchangeMem> mem;
   DBuf<int> out;
-  bar.alloc(1);
+  mem.alloc(1);
   out.alloc(4);
-  CUDA_CHECK(cudaMemsetAsync(bar.p, 0, sizeof(unsigned long long), ctx->stream));
+  CUDA_CHECK(cudaMemsetAsync(mem.p, 0, mem.bytes(), ctx->stream));
   CUDA_CHECK(cudaMemsetAsync(out.p, 0xff, 4 * sizeof(int), ctx->stream));
-  k_wait_limits<<<1, SPMV_THREADS, 0, ctx->stream>>>(bar.p, limit, out.p);
+  k_wait_limits<<<1, SPMV_THREADS, 0, ctx->stream>>>(mem.p, limit, out.p);
   LAUNCH_CHECK(ctx);
   CUDA_CHECK(cudaMemcpyAsync(results_host, out.p, 4 * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
@@ -2740,16 +2514,17 @@ void check_wait_limits_impl(fcu_ctx ctx, unsigned limit, int* results_host) {
 
 void time_pcg_impl(fcu_matrix m, int precision, i64 iters, int reps, size_t flush_bytes, double* ms,
                    double* bytes) {
-  if (!persistent_capable(m)) fail(FCU_ERR_UNSUPPORTED, "the persistent loop runs on 3x3-block point-Jacobi systems");
+  if (m->bs != 3 || m->bdinv.p)
+    fail(FCU_ERR_UNSUPPORTED, "the persistent loop is timed on 3x3-block point-Jacobi systems");
   const bool mixed = precision == FCU_MIXED;
   if (mixed && !m->val32.p) fail(FCU_ERR_BAD_ARG, "matrix has no FP32 copy");
   if (mixed && m->missing_diag) fail(FCU_ERR_UNSUPPORTED, "the mixed operator needs every diagonal block");
   fcu_ctx ctx = m->ctx;
   Workspace* w = ensure_ws(m, mixed);
-  if (!w->bar.p) w->bar.alloc(1);
+  const LoopPlan* plan = loop_plan(m, w, mixed);
+  if (!plan) fail(FCU_ERR_UNSUPPORTED, "rows too long for the persistent loop");
   ensure_inv_diag(m, w);
   if (mixed) build_rowsum32(m);
-  tune_spmv(m, w, mixed);
   const i64 n = m->n;
   k_fill_value<<<grid_for(n, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(w->b.p, n, 1.0);
   LAUNCH_CHECK(ctx);
@@ -2780,18 +2555,11 @@ void time_pcg_impl(fcu_matrix m, int precision, i64 iters, int reps, size_t flus
     else
       DISPATCH_ROWS(m->bs, w->vpr, w->grid, K_INIT64, m->row_ptr, m->col_idx, m->val64.p, m->nnodes, w->x.p, w->b.p,
                     w->invd.p, w->r.p, w->z64.p, w->pa64.p, n, w->st.p, w->partials.p);
-    pack_zp(m, w, mixed, true);
     k_flush_read<<<fgrid, 256, 0, ctx->stream>>>(reinterpret_cast<const uint4*>(flush.p), (i64)(flush_bytes / 16),
                                                  sink.p);
     CUDA_CHECK(cudaGetLastError());
-    CUDA_CHECK(cudaMemsetAsync(w->bar.p, 0, sizeof(unsigned long long), ctx->stream));
     CUDA_CHECK(cudaEventRecord(e0, ctx->stream));
-    if (mixed) {
-      if (tile_rows(4) == 64) launch_persistent_tr<true, float, 64>(m, w, m->val32.p, w->zp32.p, w->ap32.p);
-      else launch_persistent_tr<true, float, 32>(m, w, m->val32.p, w->zp32.p, w->ap32.p);
-    } else {
-      launch_persistent_tr<false, double, 32>(m, w, m->val64.p, w->zp64.p, w->ap64.p);
-    }
+    launch_persistent(m, w, *plan, mixed);
     CUDA_CHECK(cudaEventRecord(e1, ctx->stream));
     CUDA_CHECK(cudaEventSynchronize(e1));
     float t = 0.f;
