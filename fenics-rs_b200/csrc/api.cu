@@ -1176,8 +1176,9 @@ int fcu_assemble_body_force(fcu_ctx ctx, fcu_space s, const double* f, double* b
     reject_node_space(s);
     if (!s || !f || !b) fail(FCU_ERR_BAD_ARG, "null argument");
     if (s->kind != FCU_SPACE_P1_VEC3) fail(FCU_ERR_BAD_ARG, "vector space only");
-    double fh[3];
-    CUDA_CHECK(cudaMemcpy(fh, f, sizeof(fh), cudaMemcpyDefault));
+    double fh[3] = {0.0, 0.0, 0.0};
+    if (is_device_ptr(f)) CUDA_CHECK(cudaMemcpy(fh, f, sizeof(fh), cudaMemcpyDefault));
+    else std::copy(f, f + 3, fh);
     DevOut<double> bo(b, s->ndofs);
     body_force_impl(s, fh, bo.p);
     bo.finish(ctx);

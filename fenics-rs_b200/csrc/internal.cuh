@@ -122,6 +122,7 @@ struct fcu_mesh_s {
   DBuf<double> coords;    // nv*dim, AoS as the reference stores Vec<[f64;DIM]>
   DBuf<int> cells;        // nc*nodes, int32
   DBuf<unsigned char> valid;  // 1 if |det J| >= 1e-14
+  DBuf<double> cell_det;  // nc: |det J| (built by the first load vector)
   i64 n_degenerate = -1;
 };
 

@@ -69,80 +69,135 @@ __global__ void k_quad_points(const double* __restrict__ X, const int* __restric
   }
 }
 
-// f at a quadrature point: from caller values, or an analytic source.
-struct SourceEval {
-  int kind;          // -1: values array; FCU_SRC_*
-  const double* fq;  // nc*nq values (kind -1)
-  double p0, p1;
-  const double* nodal;  // FCU_SRC_NODAL: values per node
-  __device__ double operator()(i64 c, int q, const double* x, int dim, const int* nodes, const double* phi, int k) const {
-    if (kind < 0) return fq[c * (dim == 2 ? 3 : 4) + q];
-    if (kind == FCU_SRC_CONSTANT) return p0;
-    if (kind == FCU_SRC_SIN_PRODUCT) {
-      double s = p0;
-      for (int d = 0; d < dim; ++d) s = s * sin(p1 * x[d]);
-      return s;
-    }
-    // FCU_SRC_NODAL: interpolate sum_j f_j phi_j(xi_q)
-    double s = 0.0;
-    for (int j = 0; j < k; ++j) s = (j == 0) ? nodal[nodes[j]] * phi[j] : s + nodal[nodes[j]] * phi[j];
-    return s;
+// |det J| of every cell, computed on a mesh's first load vector and kept with
+// it (8 bytes a cell; the geometry does not change): a P2 load would otherwise
+// form it ten times per cell, once for each of its dofs.
+template <int DIM>
+__global__ void k_cell_det(const double* __restrict__ X, const int* __restrict__ cells, i64 nc,
+                           double* __restrict__ det) {
+  for (i64 c = blockIdx.x * (i64)blockDim.x + threadIdx.x; c < nc; c += (i64)gridDim.x * blockDim.x) {
+    int v[4];
+#pragma unroll
+    for (int j = 0; j <= DIM; ++j) v[j] = cells[(DIM + 1) * c + j];
+    if (DIM == 3) det[c] = fabs(tet_geometry(X, v).det);
+    else det[c] = fabs(tri_geometry(X, v).det);
   }
-};
+}
 
-// assemble_rhs_2d/3d and the P2 load: one thread per dof, summing its cells'
-// local loads in ascending cell order.
+// Basis values at point q of the load rule, the K functions of the space.
 template <int DIM, int K>
-__global__ void k_rhs_gather(const int* __restrict__ contrib_ptr, const int* __restrict__ contrib,
-                             const int* __restrict__ cn, const int* __restrict__ cells, const double* __restrict__ X,
-                             SourceEval f, i64 nn, double* __restrict__ b) {
-  for (i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x; i < nn; i += (i64)gridDim.x * blockDim.x) {
-    double acc = 0.0;
-    for (int t = contrib_ptr[i]; t < contrib_ptr[i + 1]; ++t) {
-      const int cc = contrib[t];
-      const i64 c = cc >> 4;
-      const int a = cc & 15;
+__device__ __forceinline__ void rule_basis(int q, double* xi, double* phi) {
+  if (DIM == 2) { xi[0] = c_tri_q2[q][0]; xi[1] = c_tri_q2[q][1]; }
+  else keast_point(q, xi);
+  if (K == 10) p2_basis(xi, phi);
+  else if (DIM == 2) { phi[0] = 1.0 - xi[0] - xi[1]; phi[1] = xi[0]; phi[2] = xi[1]; }
+  else { phi[0] = 1.0 - xi[0] - xi[1] - xi[2]; phi[1] = xi[0]; phi[2] = xi[1]; phi[3] = xi[2]; }
+}
+
+// A source that varies over the cells, evaluated once per cell and point:
+// FCU_SRC_SIN_PRODUCT at the physical point, FCU_SRC_NODAL as sum_j f_j phi_j.
+template <int DIM, int K>
+__global__ void k_cell_source(const int* __restrict__ cn, const int* __restrict__ cells, const double* __restrict__ X,
+                              int kind, double p0, double p1, const double* __restrict__ nodal, i64 nc,
+                              double* __restrict__ fq) {
+  constexpr int NQ = DIM == 2 ? 3 : 4;
+  for (i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x; t < nc * NQ; t += (i64)gridDim.x * blockDim.x) {
+    const i64 c = t / NQ;
+    const int q = (int)(t - c * NQ);
+    double xi[3], phi[K];
+    rule_basis<DIM, K>(q, xi, phi);
+    double s;
+    if (kind == FCU_SRC_SIN_PRODUCT) {
       int v[4];
       for (int j = 0; j <= DIM; ++j) v[j] = cells[(DIM + 1) * c + j];
-      double detj;
-      if (DIM == 3) detj = fabs(tet_geometry(X, v).det);
-      else detj = fabs(tri_geometry(X, v).det);
-      int nodes[K];
-      for (int j = 0; j < K; ++j) nodes[j] = cn[K * c + j];
-      double lb = 0.0;
-      const int nq = DIM == 2 ? 3 : 4;
-      for (int q = 0; q < nq; ++q) {
-        double xi[3], phi[K];
-        if (DIM == 2) { xi[0] = c_tri_q2[q][0]; xi[1] = c_tri_q2[q][1]; }
-        else keast_point(q, xi);
-        if (K == 10) p2_basis(xi, phi);
-        else if (DIM == 2) { phi[0] = 1.0 - xi[0] - xi[1]; phi[1] = xi[0]; phi[2] = xi[1]; }
-        else { phi[0] = 1.0 - xi[0] - xi[1] - xi[2]; phi[1] = xi[0]; phi[2] = xi[1]; phi[3] = xi[2]; }
-        double x[3] = {0.0, 0.0, 0.0};
-        if (f.kind == FCU_SRC_SIN_PRODUCT) phys_point(X, v, DIM, xi, x);
-        const double fv = f(c, q, x, DIM, nodes, phi, K);
-        const double w = DIM == 2 ? 1.0 / 6.0 : 1.0 / 24.0;
-        lb += w * detj * fv * phi[a];
+      double x[3];
+      phys_point(X, v, DIM, xi, x);
+      s = p0;
+      for (int d = 0; d < DIM; ++d) s = s * sin(p1 * x[d]);
+    } else {
+      s = 0.0;
+      for (int j = 0; j < K; ++j) {
+        const double f = nodal[cn[K * c + j]];
+        s = (j == 0) ? f * phi[j] : s + f * phi[j];
       }
-      acc += lb;
+    }
+    fq[t] = s;
+  }
+}
+
+// assemble_rhs_2d/3d and the P2 load: one thread per dof, summing its cells'
+// local loads in ascending cell order. CONST: f = p0, else from fq. Bound by
+// the gathers of the list: four cells' entries and determinants are fetched
+// before they are added (in list order). P2 cube 64^3, f = const: 856 us with
+// geometry and basis per (dof, cell), 48 us.
+template <int DIM, int K, bool CONST>
+__global__ void __launch_bounds__(256) k_rhs_gather(const int* __restrict__ contrib_ptr,
+                                                    const int* __restrict__ contrib, const double* __restrict__ det,
+                                                    const double* __restrict__ fq, double p0, i64 nn,
+                                                    double* __restrict__ b) {
+  constexpr int NQ = DIM == 2 ? 3 : 4, U = 4;
+  __shared__ double phi_s[NQ][K];
+  if (threadIdx.x < NQ) {
+    double xi[3], phi[K];
+    rule_basis<DIM, K>(threadIdx.x, xi, phi);
+    for (int j = 0; j < K; ++j) phi_s[threadIdx.x][j] = phi[j];
+  }
+  __syncthreads();
+  const double w = DIM == 2 ? 1.0 / 6.0 : 1.0 / 24.0;
+  for (i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x; i < nn; i += (i64)gridDim.x * blockDim.x) {
+    double acc = 0.0;
+    const int t1 = contrib_ptr[i + 1];
+    for (int t = contrib_ptr[i]; t < t1; t += U) {
+      int cc[U];
+      double d[U], f[U][CONST ? 1 : NQ];
+#pragma unroll
+      for (int u = 0; u < U; ++u) cc[u] = t + u < t1 ? contrib[t + u] : -1;
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (cc[u] >= 0) {
+          d[u] = det[cc[u] >> 4];
+          if (CONST) f[u][0] = p0;
+          else
+            for (int q = 0; q < NQ; ++q) f[u][CONST ? 0 : q] = fq[(i64)(cc[u] >> 4) * NQ + q];
+        }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (cc[u] >= 0) {
+          double lb = 0.0;
+#pragma unroll
+          for (int q = 0; q < NQ; ++q) lb += w * d[u] * f[u][CONST ? 0 : q] * phi_s[q][cc[u] & 15];
+          acc += lb;
+        }
     }
     b[i] = acc;
   }
 }
 
 // assemble_elasticity_body_force_3d (elasticity.rs:153-185)
-__global__ void k_body_force(const int* __restrict__ contrib_ptr, const int* __restrict__ contrib,
-                             const int* __restrict__ cells, const double* __restrict__ X, double f0, double f1,
-                             double f2, i64 nv, double* __restrict__ b) {
+__global__ void __launch_bounds__(256) k_body_force(const int* __restrict__ contrib_ptr,
+                                                    const int* __restrict__ contrib, const double* __restrict__ det,
+                                                    double f0, double f1, double f2, i64 nv,
+                                                    double* __restrict__ b) {
+  constexpr int U = 4;
   for (i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x; i < nv; i += (i64)gridDim.x * blockDim.x) {
     double a0 = 0.0, a1 = 0.0, a2 = 0.0;
-    for (int t = contrib_ptr[i]; t < contrib_ptr[i + 1]; ++t) {
-      const i64 c = contrib[t] >> 4;
-      int v[4] = {cells[4 * c], cells[4 * c + 1], cells[4 * c + 2], cells[4 * c + 3]};
-      const double vol = (1.0 / 6.0) * fabs(tet_geometry(X, v).det);
-      a0 += f0 * (vol * 0.25);
-      a1 += f1 * (vol * 0.25);
-      a2 += f2 * (vol * 0.25);
+    const int t1 = contrib_ptr[i + 1];
+    for (int t = contrib_ptr[i]; t < t1; t += U) {
+      int cc[U];
+      double d[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) cc[u] = t + u < t1 ? contrib[t + u] : -1;
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (cc[u] >= 0) d[u] = det[cc[u] >> 4];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (cc[u] >= 0) {
+          const double vol = (1.0 / 6.0) * d[u];
+          a0 += f0 * (vol * 0.25);
+          a1 += f1 * (vol * 0.25);
+          a2 += f2 * (vol * 0.25);
+        }
     }
     b[3 * i] = a0;
     b[3 * i + 1] = a1;
@@ -329,28 +384,56 @@ void quadrature_points_impl(fcu_space s, double* out_dev) {
   LAUNCH_CHECK(ctx);
 }
 
-void rhs_impl(fcu_space s, int kind, const double* fq_dev, double p0, double p1, const double* nodal_dev, double* b_dev) {
+static const double* cell_det(fcu_mesh m) {
+  fcu_ctx ctx = m->ctx;
+  if (!m->cell_det.p && m->nc) {
+    m->cell_det.alloc(m->nc);
+    const unsigned g = grid_for(m->nc, 128, ctx->num_sms * 16);
+    if (m->dim == 3) k_cell_det<3><<<g, 128, 0, ctx->stream>>>(m->coords.p, m->cells.p, m->nc, m->cell_det.p);
+    else k_cell_det<2><<<g, 128, 0, ctx->stream>>>(m->coords.p, m->cells.p, m->nc, m->cell_det.p);
+    LAUNCH_CHECK(ctx);
+  }
+  return m->cell_det.p;
+}
+
+template <int DIM, int K>
+static void rhs_space(fcu_space s, int kind, const double* fq_dev, double p0, double p1, const double* nodal_dev,
+                      double* b_dev) {
   fcu_ctx ctx = s->ctx;
   fcu_mesh m = s->mesh;
-  SourceEval f{kind, fq_dev, p0, p1, nodal_dev};
-  const unsigned g = grid_for(s->nnodes, 128, ctx->num_sms * 16);
-  if (s->kind == FCU_SPACE_P2)
-    k_rhs_gather<3, 10><<<g, 128, 0, ctx->stream>>>(s->contrib_ptr.p, s->contrib.p, s->cell_nodes.p, m->cells.p,
-                                                    m->coords.p, f, s->nnodes, b_dev);
-  else if (m->dim == 3)
-    k_rhs_gather<3, 4><<<g, 128, 0, ctx->stream>>>(s->contrib_ptr.p, s->contrib.p, s->cell_nodes.p, m->cells.p,
-                                                   m->coords.p, f, s->nnodes, b_dev);
-  else
-    k_rhs_gather<2, 3><<<g, 128, 0, ctx->stream>>>(s->contrib_ptr.p, s->contrib.p, s->cell_nodes.p, m->cells.p,
-                                                   m->coords.p, f, s->nnodes, b_dev);
+  constexpr int NQ = DIM == 2 ? 3 : 4;
+  const double* det = cell_det(m);
+  const unsigned g = grid_for(s->nnodes, 256, ctx->num_sms * 16);
+  if (kind == FCU_SRC_CONSTANT) {
+    k_rhs_gather<DIM, K, true><<<g, 256, 0, ctx->stream>>>(s->contrib_ptr.p, s->contrib.p, det, nullptr, p0,
+                                                           s->nnodes, b_dev);
+    LAUNCH_CHECK(ctx);
+    return;
+  }
+  DBuf<double> fq;
+  if (kind >= 0 && m->nc) {
+    fq.alloc(m->nc * NQ);
+    k_cell_source<DIM, K><<<grid_for(m->nc * NQ, 128, ctx->num_sms * 16), 128, 0, ctx->stream>>>(
+        s->cell_nodes.p, m->cells.p, m->coords.p, kind, p0, p1, nodal_dev, m->nc, fq.p);
+    LAUNCH_CHECK(ctx);
+  }
+  k_rhs_gather<DIM, K, false><<<g, 256, 0, ctx->stream>>>(s->contrib_ptr.p, s->contrib.p, det,
+                                                          kind >= 0 ? fq.p : fq_dev, p0, s->nnodes, b_dev);
   LAUNCH_CHECK(ctx);
+}
+
+void rhs_impl(fcu_space s, int kind, const double* fq_dev, double p0, double p1, const double* nodal_dev, double* b_dev) {
+  if (s->kind == FCU_SPACE_P2) rhs_space<3, 10>(s, kind, fq_dev, p0, p1, nodal_dev, b_dev);
+  else if (s->mesh->dim == 3) rhs_space<3, 4>(s, kind, fq_dev, p0, p1, nodal_dev, b_dev);
+  else rhs_space<2, 3>(s, kind, fq_dev, p0, p1, nodal_dev, b_dev);
 }
 
 void body_force_impl(fcu_space s, const double* f, double* b_dev) {
   fcu_ctx ctx = s->ctx;
   fcu_mesh m = s->mesh;
-  k_body_force<<<grid_for(m->nv, 128, ctx->num_sms * 16), 128, 0, ctx->stream>>>(
-      s->contrib_ptr.p, s->contrib.p, m->cells.p, m->coords.p, f[0], f[1], f[2], m->nv, b_dev);
+  const double* det = cell_det(m);
+  k_body_force<<<grid_for(m->nv, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(
+      s->contrib_ptr.p, s->contrib.p, det, f[0], f[1], f[2], m->nv, b_dev);
   LAUNCH_CHECK(ctx);
 }
 
