@@ -1099,6 +1099,50 @@ __global__ void k_spmv_plain(const int* __restrict__ rp, const int* __restrict__
   spmv_rows<BS, VPR, false, double>(rp, ci, val, nrows, XPlain<double>{x}, em);
 }
 
+// Scalar rows of medium length (8 to 64 entries on average): VPR lanes per
+// row (loop_lanes), each fetching eight entries' columns and values and then
+// their operands together, so a row of up to 8 VPR entries costs two dependent
+// round trips. No shared memory: the whole L1 serves the operand gathers.
+// Bound by the gathers' L1 wavefronts and HBM. P2 matrix of the 64^3 cube
+// (61M entries, 4 lanes): 156 us, 219 us with the CSR-stream kernel; P1 matrix
+// of the 96^3 cube (2 lanes): 33.6 us. Other shapes measured there: 8 lanes of
+// 4 entries 172 / 55.6 us, 4 of 4 172 / 37.0, 8 of 2 169 / 46.8, 2 of 8 183 /
+// 33.6, 4 of 8 156 / 43.7.
+template <int VPR>
+__global__ void __launch_bounds__(256) k_spmv_medium(const int* __restrict__ rp, const int* __restrict__ ci,
+                                                     const double* __restrict__ val, i64 nrows,
+                                                     const double* __restrict__ x, double* __restrict__ y) {
+  grid_dep_sync();
+  constexpr int E = 8;
+  const int lane = threadIdx.x & 31, sub = lane % VPR;
+  constexpr int RPW = 32 / VPR;
+  const i64 gw = (blockIdx.x * (i64)blockDim.x + threadIdx.x) >> 5, nw = ((i64)gridDim.x * blockDim.x) >> 5;
+  for (i64 base = gw * RPW; base < nrows; base += nw * RPW) {
+    const i64 row = base + lane / VPR;
+    double s = 0.0;
+    if (row < nrows) {
+      const int e1 = rp[row + 1];
+      for (int q = rp[row] + sub; q < e1; q += E * VPR) {
+        int c[E];
+        double v[E], g[E];
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+          const bool in = q + e * VPR < e1;
+          c[e] = in ? __ldcs(ci + q + e * VPR) : -1;
+          v[e] = in ? __ldcs(val + q + e * VPR) : 0.0;
+        }
+#pragma unroll
+        for (int e = 0; e < E; ++e) g[e] = c[e] >= 0 ? x[c[e]] : 0.0;
+#pragma unroll
+        for (int e = 0; e < E; ++e) s += v[e] * g[e];
+      }
+    }
+#pragma unroll
+    for (int o = VPR / 2; o > 0; o >>= 1) s += __shfl_xor_sync(FULL, s, o);
+    if (row < nrows && sub == 0) y[row] = s;
+  }
+}
+
 // ---------------------------------------------------------------------------
 // CSR-stream SpMV for scalar matrices with short rows. CTA-sized row blocks
 // (at most STREAM_ROWS rows and STREAM_NNZ entries, built once per matrix)
@@ -2157,6 +2201,18 @@ void invalidate_graphs(fcu_matrix m) {
 
 void spmv_impl(fcu_matrix m, const double* x_dev, double* y_dev) {
   fcu_ctx ctx = m->ctx;
+  const double mean = m->nnodes ? (double)m->nnzb / (double)m->nnodes : 0.0;
+  if (m->bs == 1 && mean > 8.0 && mean <= 64.0) {
+    const int v = loop_lanes(mean);
+    auto go = [&](auto kern) {
+      launch_pdl_cfg(ctx, kern, (int)grid_for(m->nnodes * v, 256, 1 << 20), 256, 0, m->row_ptr, m->col_idx,
+                     m->val64.p, m->nnodes, x_dev, y_dev);
+    };
+    if (v == 2) go(k_spmv_medium<2>);
+    else if (v == 4) go(k_spmv_medium<4>);
+    else go(k_spmv_medium<8>);
+    return;
+  }
   if (use_stream_spmv(m)) {
     ensure_row_blocks(m);
     launch_pdl_cfg(ctx, k_spmv_stream_plain, stream_grid_for(ctx, m->nrowblk, k_spmv_stream_plain), STREAM_THREADS, 0, m->row_ptr, m->col_idx,
