@@ -6,21 +6,22 @@
 // the library's pattern, assembly, load-vector and Dirichlet kernels build
 // the whole batch in one pass each, and block i is rows [off[i], off[i+1]).
 //
-// One persistent launch solves the batch. Each thread-block cluster (1 to 8
-// CTAs) takes the next instance from a queue ordered by estimated cost
-// (largest first) and runs that instance's whole PCG: the cluster's CTAs own
-// contiguous shares of its rows, phases are separated by cluster barriers,
-// and every reduction sums the CTAs' partials through distributed shared
-// memory in rank order, so instances converge, stop and report independently
-// and no grid-wide synchronisation exists. The arithmetic per instance is
-// that of the library's single-system PCG (cg.rs:40-149 for FP64; for mixed,
-// FP32 difference-form operator with FP64 r, x and dots and FP64 residual
-// replacement). The launch is captured in a CUDA graph together with the
-// queue reset, and the graph is replayed on later solves. Lanes per row,
-// threads per CTA and CTAs per cluster are picked by timing the candidates on
-// the batch itself (first solve of a matrix and precision), unless
-// FCU_BATCH_VPR / FCU_BATCH_THREADS / FCU_BATCH_CLUSTER fix them; a single
-// system (the small-system path of the PCG) takes a shape fixed by rule.
+// Each instance is solved by one thread-block cluster, whose CTAs own contiguous
+// shares of its rows and sum their partials through distributed shared memory
+// in rank order, so instances converge, stop and report independently and no
+// grid-wide synchronisation exists. The arithmetic per instance is that of the
+// library's single-system PCG (cg.rs:40-149 for FP64; for mixed, FP32
+// difference-form operator with FP64 r, x and dots and FP64 residual
+// replacement). Two forms: the resident one holds the instance on chip
+// (clusters of 1 to 16 CTAs, one launch per cluster size, the launches side by
+// side); the streaming one, for instances that do not fit, reads its data from
+// memory each iteration (clusters of 1 to 8 that take instances from a queue in
+// order of estimated cost). Several launches are captured in a CUDA graph, which
+// later solves replay. The streaming form's lanes per row, threads per CTA and
+// CTAs per cluster are picked by timing the candidates on its instances (first
+// solve of a matrix and precision), unless FCU_BATCH_VPR / FCU_BATCH_THREADS /
+// FCU_BATCH_CLUSTER fix them; a single system (the small-system path of the
+// PCG) takes a shape fixed by rule.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
@@ -402,6 +403,313 @@ __global__ void __launch_bounds__(BT, 1024 / BT) k_batch_pcg(BatchArgs a) {
   }
 }
 
+// ---------------------------------------------------------------------------
+// Resident form: a cluster of 1 to 16 CTAs holds its whole instance on chip for
+// the duration of its PCG. Each CTA owns a contiguous share of the rows; the
+// share's matrix entries lie in shared memory (ELL: entry e of all rows
+// together, two 16-bit columns to a word, relative to the CTA's window of the
+// direction), x, r and D^-1 in registers (RM rows per thread), and the window
+// of p (own rows plus the band on either side) in shared memory. An iteration
+// touches no global memory; it has two cluster barriers:
+//   p = z + beta p over the window (z of other CTAs' rows read from their
+//   shared memory), Ap from shared memory           -> p.Ap over the cluster
+//   x, r updated in registers, z stored             -> r.z and r.r
+// What bounds it: instruction issue of the product (29k warp instructions per SM
+// and iteration with full shares, 50 % of the issue slots; 5.1k of them shared
+// loads) and the two cluster barriers of 1.1 us. A 257^2 instance takes 6.9 us
+// per iteration on 16 SMs; the streaming form, bound by chains of L2 loads,
+// took 100 us on its two. 256 instances of 32^2 to 256^2 cells, mixed, to 1e-8:
+// 108 -> 61 ms (FP64 140 -> 92); one 64^2: 1.67 -> 1.05 ms. One row at a time
+// per thread: sums of three rows side by side, and shapes with fewer rows on
+// more threads, spilled and took 5 to 30 % longer. The diagonal is entry 0, on
+// the row's own operand, so that no entry has to be compared with its row.
+// Rows that do not fit (FP64, the largest instances) stay in global memory and
+// are read from there.
+// ---------------------------------------------------------------------------
+
+constexpr int RNT = 512;        // threads per CTA
+constexpr int RM = 9;           // rows per thread, at most
+constexpr int RMAXC = 16;       // CTAs per cluster, at most
+constexpr int RMAX_WIDTH = 32;  // entries per row, at most
+
+struct ResidentInfo {
+  int width;  // entries of the longest row, a diagonal slot included
+  int band;   // largest |column - row|
+  int cap;    // rows of a CTA's share held in shared memory
+  int share;  // rows per CTA
+};
+
+// Byte offsets of a CTA's shared memory: the window of p first (the stored
+// columns are byte offsets into it), own z, the matrix.
+struct ResidentLayout {
+  size_t z, val, col, end;
+  __host__ __device__ ResidentLayout(int wv, int share, int band, int width, int cap) {
+    auto al = [](size_t x) { return (x + 15) & ~(size_t)15; };
+    z = al(((size_t)share + 2 * (size_t)band) * wv);
+    val = z + al((size_t)share * wv);
+    col = val + al((size_t)width * cap * wv);
+    end = col + al((size_t)((width + 1) / 2) * cap * 4);
+  }
+};
+
+// NV sums over the cluster: the CTA's sum goes to every CTA's slots before the
+// cluster barrier, after which each warp adds its own copy in rank order (a
+// fixed shuffle tree), so every thread of every CTA has the same totals.
+template <int NV>
+__device__ __forceinline__ void resident_sum(double (&v)[NV], double (*sh)[RNT / 32], double (*slots)[2][RMAXC],
+                                             int& parity, cg::cluster_group& cl, unsigned ncl, unsigned rank) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+  for (int j = 0; j < NV; ++j) {
+    const double x = bwarp_sum(v[j]);
+    if (lane == 0) sh[j][w] = x;
+  }
+  __syncthreads();
+  if (w == 0) {
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+      const double x = bwarp_sum(lane < RNT / 32 ? sh[j][lane] : 0.0);
+      if (lane < (int)ncl) *cl.map_shared_rank(&slots[parity][j][rank], lane) = x;
+    }
+  }
+  if (ncl > 1) cl.sync();
+  else __syncthreads();
+#pragma unroll
+  for (int j = 0; j < NV; ++j) v[j] = bwarp_sum(lane < (int)ncl ? slots[parity][j][lane] : 0.0);
+  parity ^= 1;
+}
+
+template <class T>
+__global__ void __launch_bounds__(RNT, 1) k_batch_resident(BatchArgs a, const int* __restrict__ list,
+                                                          const ResidentInfo* __restrict__ info, int count,
+                                                          int* __restrict__ next) {
+  constexpr bool MIXED = sizeof(T) == 4;
+  extern __shared__ __align__(16) unsigned char res_smem[];
+  __shared__ double sh[2][RNT / 32];
+  __shared__ double slots[2][2][RMAXC];
+  __shared__ int turn;
+  cg::cluster_group cl = cg::this_cluster();
+  const unsigned ncl = cl.num_blocks(), rank = cl.block_rank();
+  int parity = 0;
+  const int tid = threadIdx.x;
+  // instances: as many as clusters at once, the others as clusters come free
+  for (int at = (int)(blockIdx.x / ncl); at < count;) {
+    const int inst = list[at];
+    const ResidentInfo in = info[inst];
+    const int r0 = (int)a.off[inst], r1 = (int)a.off[inst + 1];
+    const int c0 = min(r0 + (int)rank * in.share, r1), c1 = min(c0 + in.share, r1);
+    const int nloc = c1 - c0;
+    const int wlo = max(r0, c0 - in.band), whi = min(r1, c1 + in.band);  // window of p
+    const int off = c0 - wlo;
+    const int lo_halo = nloc > 0 ? off : 0, hi_halo = nloc > 0 ? whi - c1 : 0;
+    const ResidentLayout L(sizeof(T), in.share, in.band, in.width, in.cap);
+    T* const pw = reinterpret_cast<T*>(res_smem);
+    T* const zs = reinterpret_cast<T*>(res_smem + L.z);
+    T* const ev = reinterpret_cast<T*>(res_smem + L.val);
+    unsigned* const ec = reinterpret_cast<unsigned*>(res_smem + L.col);
+    const T* const vals = MIXED ? reinterpret_cast<const T*>(a.val32) : reinterpret_cast<const T*>(a.val64);
+
+    // the matrix: the diagonal slot first (its column is not looked up), then the
+    // row's other entries; unused ones have weight 0 on the row's own operand
+    for (int i = tid; i < min(nloc, in.cap); i += RNT) {
+      const int a1 = a.rp[c0 + i + 1];
+      int q = a.rp[c0 + i];
+      const unsigned self = (unsigned)(off + i) * (unsigned)sizeof(T);
+      T d = T(0);
+      auto next = [&](T& v) {  // the next off-diagonal entry: weight, offset of its p
+        for (; q < a1; ++q) {
+          const int c = a.ci[q] - wlo;
+          v = vals[q];
+          if (c != off + i) {
+            ++q;
+            return (unsigned)c * (unsigned)sizeof(T);
+          }
+          d += v;
+        }
+        v = T(0);
+        return self;
+      };
+      for (int e = 0; e < in.width; e += 2) {
+        T v0, v1;
+        const unsigned k0 = e ? next(v0) : self, k1 = next(v1);
+        ec[(e >> 1) * in.cap + i] = k0 | (k1 << 16);
+        if (e) ev[e * in.cap + i] = v0;
+        if (e + 1 < in.width) ev[(e + 1) * in.cap + i] = v1;
+      }
+      while (q < a1) {  // only the diagonal can be left
+        T v;
+        next(v);
+      }
+      ev[i] = d;
+    }
+    // x0 = 0: r = b, z = D^-1 r, p = 0 (cg.rs:79-90)
+    double xv[RM], rv[RM], dv[RM];
+    double v2[2] = {0.0, 0.0};
+#pragma unroll
+    for (int k = 0; k < RM; ++k) {
+      const int i = tid + k * RNT;
+      xv[k] = 0.0;
+      rv[k] = i < nloc ? a.b[c0 + i] : 0.0;
+      dv[k] = i < nloc ? a.invd[c0 + i] : 0.0;
+      if (i < nloc) {
+        const double zi = rv[k] * dv[k];
+        zs[i] = (T)zi;
+        v2[0] += rv[k] * zi;
+        v2[1] += rv[k] * rv[k];
+      }
+    }
+    for (int j = tid; j < whi - wlo; j += RNT) pw[j] = T(0);
+    resident_sum<2>(v2, sh, slots, parity, cl, ncl, rank);
+    double rz = v2[0], rr = v2[1];
+    const double bnorm = sqrt(rr);
+    double maxr = bnorm, beta = 0.0;
+    i64 iter = 0, updates = 0;
+    int status = FCU_ERR_NO_CONVERGENCE;
+    if (bnorm < a.tol || (bnorm > 0.0 && bnorm / bnorm < a.tol)) status = FCU_OK;
+    while (status != FCU_OK && iter < a.max_iter) {
+      // p = z + beta p over the window
+      const T bt = (T)beta;
+      for (int i = tid; i < nloc; i += RNT) pw[off + i] = fma(bt, pw[off + i], zs[i]);
+      for (int h = tid; h < lo_halo + hi_halo; h += RNT) {
+        const int j = h < lo_halo ? h : h + nloc;
+        const int g = wlo + j - r0;
+        const int q = g / in.share;
+        const T z = *cl.map_shared_rank(zs + (g - q * in.share), q);
+        pw[j] = fma(bt, pw[j], z);
+      }
+      __syncthreads();
+      // Ap and p.Ap
+      double v1[1] = {0.0};
+      T apv[RM];
+#pragma unroll
+      for (int k = 0; k < RM; ++k) {
+        const int i = tid + k * RNT;
+        apv[k] = T(0);
+        if (i < nloc) {
+          // the diagonal slot on its own operand; mixed: the others act on
+          // differences
+          const T own = pw[off + i];
+          T s;
+          auto add = [&](T v, unsigned at) {  // at: byte offset of the column's p
+            const T y = *reinterpret_cast<const T*>(res_smem + at);
+            s += v * (MIXED ? y - own : y);
+          };
+          if (i < in.cap) {
+            const unsigned* pc = ec + i;
+            const T* pv = ev + i;
+            s = pv[0] * own;
+            if (in.width > 1) add(pv[in.cap], *pc >> 16);
+            int e = 2;
+#pragma unroll 2
+            for (; e + 1 < in.width; e += 2) {
+              pc += in.cap;
+              pv += 2 * in.cap;
+              const unsigned cc = *pc;
+              add(pv[0], cc & 0xffffu);
+              add(pv[in.cap], cc >> 16);
+            }
+            if (e < in.width) add(pv[2 * in.cap], pc[in.cap] & 0xffffu);
+          } else {
+            const int a1 = a.rp[c0 + i + 1];
+            s = T(0);
+            for (int q = a.rp[c0 + i]; q < a1; ++q) {
+              const int c = a.ci[q] - wlo;
+              s += vals[q] * (MIXED && c != off + i ? pw[c] - own : pw[c]);
+            }
+          }
+          apv[k] = s;
+          v1[0] += (double)own * (double)s;
+        }
+      }
+      resident_sum<1>(v1, sh, slots, parity, cl, ncl, rank);
+      if (fabs(v1[0]) < 1e-30) {  // cg.rs:102-107
+        iter += 1;
+        status = FCU_ERR_BREAKDOWN;
+        break;
+      }
+      const double alpha = rz / v1[0];
+      // x += alpha p, r -= alpha Ap, z = D^-1 r
+      v2[0] = v2[1] = 0.0;
+#pragma unroll
+      for (int k = 0; k < RM; ++k) {
+        const int i = tid + k * RNT;
+        if (i < nloc) {
+          xv[k] += alpha * (double)pw[off + i];
+          rv[k] -= alpha * (double)apv[k];
+          const double zi = rv[k] * dv[k];
+          zs[i] = (T)zi;
+          v2[0] += rv[k] * zi;
+          v2[1] += rv[k] * rv[k];
+        }
+      }
+      resident_sum<2>(v2, sh, slots, parity, cl, ncl, rank);
+      iter += 1;
+      rr = v2[1];
+      const double res = sqrt(rr);
+      const double rel = bnorm > 0.0 ? res / bnorm : res;
+      if (!MIXED) {
+        if (rel < a.tol) {
+          status = FCU_OK;
+          break;
+        }
+      } else if (rel < a.tol || res < a.delta * maxr) {
+        // residual replacement with the FP64 matrix: r = b - A64 x, z = D^-1 r
+#pragma unroll
+        for (int k = 0; k < RM; ++k)
+          if (tid + k * RNT < nloc) a.x[c0 + tid + k * RNT] = xv[k];
+        if (ncl > 1) cl.sync();
+        else __syncthreads();
+        v2[0] = v2[1] = 0.0;
+#pragma unroll
+        for (int k = 0; k < RM; ++k) {
+          const int i = tid + k * RNT;
+          if (i < nloc) {
+            double s = 0.0;
+            const int a1 = a.rp[c0 + i + 1];
+            for (int q = a.rp[c0 + i]; q < a1; ++q) s += a.val64[q] * __ldcg(a.x + a.ci[q]);
+            rv[k] = a.b[c0 + i] - s;
+            const double zi = rv[k] * dv[k];
+            zs[i] = (T)zi;
+            v2[0] += rv[k] * zi;
+            v2[1] += rv[k] * rv[k];
+          }
+        }
+        resident_sum<2>(v2, sh, slots, parity, cl, ncl, rank);
+        updates += 1;
+        rr = v2[1];
+        const double res2 = sqrt(rr);
+        const double rel2 = bnorm > 0.0 ? res2 / bnorm : res2;
+        if (rel2 < a.tol) {
+          status = FCU_OK;
+          break;
+        }
+        maxr = res2;
+      }
+      beta = v2[0] / rz;
+      rz = v2[0];
+    }
+#pragma unroll
+    for (int k = 0; k < RM; ++k)
+      if (tid + k * RNT < nloc) a.x[c0 + tid + k * RNT] = xv[k];
+    if (rank == 0 && tid == 0) {
+      a.iters[inst] = iter;
+      a.updates[inst] = updates;
+      a.relres[inst] = bnorm > 0.0 ? sqrt(rr) / bnorm : sqrt(rr);
+      a.resid[inst] = sqrt(rr);
+      a.status[inst] = status;
+    }
+    if ((int)(gridDim.x / ncl) >= count) break;
+    if (rank == 0 && tid < (int)ncl) {
+      int v = 0;
+      if (tid == 0) v = (int)(gridDim.x / ncl) + atomicAdd(next, 1);
+      v = __shfl_sync(__activemask(), v, 0);
+      *cl.map_shared_rank(&turn, tid) = v;
+    }
+    cl.sync();
+    at = turn;
+  }
+}
+
 // D^-1 from the diagonal slots (cg.rs:52-64: 1 when |a_kk| <= 1e-15).
 __global__ void k_batch_invd(const int* __restrict__ diag_pos, const double* __restrict__ val, i64 n,
                              double* __restrict__ invd) {
@@ -412,16 +720,43 @@ __global__ void k_batch_invd(const int* __restrict__ diag_pos, const double* __r
   }
 }
 
-// Every row of block i must only reference columns of block i.
+// Every row of block i must only reference columns of block i; its entries,
+// longest row and bandwidth (info[4 i ..]). Blocks (i, *) share instance i.
 __global__ void k_batch_check(const int* __restrict__ rp, const int* __restrict__ ci, const i64* __restrict__ off,
-                              int nb, int* __restrict__ bad) {
+                              int nb, int* __restrict__ bad, int* __restrict__ info) {
   const int inst = blockIdx.x;
   if (inst >= nb) return;
   const i64 r0 = off[inst], r1 = off[inst + 1];
-  for (i64 row = r0 + threadIdx.x; row < r1; row += blockDim.x)
-    for (int q = rp[row]; q < rp[row + 1]; ++q)
-      if (ci[q] < r0 || ci[q] >= r1) atomicExch(bad, 1);
+  int nnz = 0, len = 0, band = 0;
+  for (i64 row = r0 + blockIdx.y * blockDim.x + threadIdx.x; row < r1; row += (i64)gridDim.y * blockDim.x) {
+    const int b = rp[row], e = rp[row + 1];
+    nnz += e - b;
+    int others = 0;
+    for (int q = b; q < e; ++q) {
+      const int c = ci[q];
+      others += c != (int)row;
+      if (c < r0 || c >= r1) atomicExch(bad, 1);
+      band = max(band, abs(c - (int)row));
+    }
+    len = max(len, others + 1);
+  }
+  nnz = __reduce_add_sync(BFULL, nnz);
+  len = __reduce_max_sync(BFULL, len);
+  band = __reduce_max_sync(BFULL, band);
+  if ((threadIdx.x & 31) == 0) {
+    atomicAdd(&info[4 * inst], nnz);
+    atomicMax(&info[4 * inst + 1], len);
+    atomicMax(&info[4 * inst + 2], band);
+  }
 }
+
+// One resident launch: the instances that take clusters of this size.
+struct ResidentClass {
+  int cluster = 1;
+  int first = 0, count = 0;  // in the class list
+  int clusters = 0;          // launched; fewer than count: they take instances in turn
+  size_t smem = 0;
+};
 
 struct BatchConfig {
   int vpr = 1;
@@ -450,7 +785,6 @@ struct BatchWorkspace {
   int nb = 0;
   std::vector<i64> off;  // host copy of the offsets
   DBuf<i64> off_d;
-  DBuf<int> order;
   DBuf<double> b, x, r, invd;
   DBuf<double> z64, p64, q64, ap64;  // q: the second direction buffer
   DBuf<float> z32, p32, q32, ap32;
@@ -458,15 +792,24 @@ struct BatchWorkspace {
   DBuf<i64> iters, updates;
   DBuf<double> relres, resid;
   DBuf<int> status;
+  std::vector<int> nnz, width, band;  // per instance: entries, longest row, bandwidth
+  std::vector<ResidentClass> classes[2];  // resident launches (FP64, FP32), then the instances left to the queue
+  DBuf<ResidentInfo> info[2];
+  DBuf<int> lists[2];                 // instances by class, the queue's last
+  DBuf<int> turns;                    // by cluster size: instances taken so far beyond the first ones
+  int nqueue[2] = {0, 0};
+  std::vector<cudaStream_t> side;     // branches of the captured launch
+  std::vector<cudaEvent_t> joins;
   BatchConfig cfg[2];
   bool tuned[2] = {false, false};
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
-  int graph_key[2] = {-1, -1};  // configuration of the captured launch
   double tol_g[2] = {0.0, 0.0};
   i64 iters_g[2] = {0, 0};
   ~BatchWorkspace() {
     for (auto& g : graph)
       if (g) cudaGraphExecDestroy(g);
+    for (auto& e : joins) cudaEventDestroy(e);
+    for (auto& t : side) cudaStreamDestroy(t);
   }
 };
 
@@ -486,8 +829,8 @@ BatchArgs make_args(fcu_matrix m, BatchWorkspace* w, bool mixed, double tol, i64
   a.val64 = m->val64.p;
   a.val32 = m->val32.p;
   a.off = w->off_d.p;
-  a.order = w->order.p;
-  a.nb = w->nb;
+  a.order = w->lists[mixed ? 1 : 0].p + (w->nb - w->nqueue[mixed ? 1 : 0]);
+  a.nb = w->nqueue[mixed ? 1 : 0];
   a.b = w->b.p;
   a.x = w->x.p;
   a.r = w->r.p;
@@ -542,13 +885,13 @@ int batch_grid(fcu_ctx ctx, BatchKernel k, const BatchConfig& c, int nb) {
   return c.cluster * std::min(nb, nclusters);
 }
 
-void launch_batch(fcu_ctx ctx, BatchWorkspace* w, BatchKernel k, const BatchConfig& c, int grid,
+void launch_batch(cudaStream_t stream, BatchWorkspace* w, BatchKernel k, const BatchConfig& c, int grid,
                   const BatchArgs& a) {
-  CUDA_CHECK(cudaMemsetAsync(w->counter.p, 0, sizeof(unsigned), ctx->stream));
+  CUDA_CHECK(cudaMemsetAsync(w->counter.p, 0, sizeof(unsigned), stream));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3((unsigned)c.threads);
-  cfg.stream = ctx->stream;
+  cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = (unsigned)c.cluster;
@@ -566,8 +909,8 @@ BatchConfig autotune(fcu_matrix m, BatchWorkspace* w, bool mixed, double tol) {
   fixed.vpr = env_int("FCU_BATCH_VPR", 0);
   fixed.threads = env_int("FCU_BATCH_THREADS", 0);
   fixed.cluster = env_int("FCU_BATCH_CLUSTER", 0);
-  if (fixed.vpr && fixed.threads && fixed.cluster && pick_kernel(mixed, fixed, w->nb) &&
-      batch_grid(m->ctx, pick_kernel(mixed, fixed, w->nb), fixed, w->nb) > 0)
+  if (fixed.vpr && fixed.threads && fixed.cluster && pick_kernel(mixed, fixed, w->nqueue[mixed ? 1 : 0]) &&
+      batch_grid(m->ctx, pick_kernel(mixed, fixed, w->nqueue[mixed ? 1 : 0]), fixed, w->nqueue[mixed ? 1 : 0]) > 0)
     return fixed;
   fcu_ctx ctx = m->ctx;
   const int vprs[3] = {1, 2, 4};
@@ -586,13 +929,13 @@ BatchConfig autotune(fcu_matrix m, BatchWorkspace* w, bool mixed, double tol) {
         c.vpr = v;
         c.threads = t;
         c.cluster = cs;
-        BatchKernel k = pick_kernel(mixed, c, w->nb);
+        BatchKernel k = pick_kernel(mixed, c, w->nqueue[mixed ? 1 : 0]);
         if (!k) continue;
-        const int grid = batch_grid(ctx, k, c, w->nb);
+        const int grid = batch_grid(ctx, k, c, w->nqueue[mixed ? 1 : 0]);
         if (grid <= 0) continue;
-        launch_batch(ctx, w, k, c, grid, a);  // warm
+        launch_batch(ctx->stream, w, k, c, grid, a);  // warm
         CUDA_CHECK(cudaEventRecord(e0, ctx->stream));
-        launch_batch(ctx, w, k, c, grid, a);
+        launch_batch(ctx->stream, w, k, c, grid, a);
         CUDA_CHECK(cudaEventRecord(e1, ctx->stream));
         CUDA_CHECK(cudaEventSynchronize(e1));
         float ms = 0.f;
@@ -606,6 +949,183 @@ BatchConfig autotune(fcu_matrix m, BatchWorkspace* w, bool mixed, double tol) {
   cudaEventDestroy(e1);
   if (best_ms >= 1e30f) fail(FCU_ERR_UNSUPPORTED, "no batched PCG configuration fits this device");
   return best;
+}
+
+// Dynamic shared memory a resident CTA may use; allows it, and clusters of 16,
+// to the kernel.
+template <class T>
+size_t resident_limit(fcu_ctx ctx) {
+  int optin = 0;
+  CUDA_CHECK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device));
+  const size_t limit = (size_t)optin - 2048;  // its static arrays
+  CUDA_CHECK(cudaFuncSetAttribute(k_batch_resident<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit));
+  CUDA_CHECK(cudaFuncSetAttribute(k_batch_resident<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  return limit;
+}
+
+template <class T>
+cudaLaunchConfig_t resident_config(fcu_ctx ctx, cudaLaunchAttribute* attr, int cluster, int count, size_t smem,
+                                   cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(cluster * count));
+  cfg.blockDim = dim3(RNT);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = (unsigned)cluster;
+  attr->val.clusterDim.y = 1;
+  attr->val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
+// Sorts the instances into resident launches by cluster size, largest cost
+// first within each, and the rest (rows long or of very different lengths, or
+// an instance larger than a cluster holds) to the queue of the streaming
+// kernel. An instance takes the smallest cluster that holds all of it on chip,
+// so that a CTA always has about as many rows to work on between barriers;
+// where none does (FP64 above about 40k rows of seven entries), the largest
+// cluster, with the rows that do not fit read from global memory. A batch that
+// would leave most SMs idle takes larger clusters.
+template <class T>
+void plan_resident(fcu_matrix m, BatchWorkspace* w, const std::vector<int>& by_cost) {
+  fcu_ctx ctx = m->ctx;
+  const int k = sizeof(T) == 4 ? 1 : 0, wv = (int)sizeof(T);
+  const size_t limit = resident_limit<T>(ctx);
+  // clusters of each size that the device runs at a time with full shared memory
+  std::array<int, RMAXC + 1>& active = ctx->batch_clusters[k];
+  if (!active[1])
+    for (int c = RMAXC; c > 0; --c) {
+      cudaLaunchAttribute attr;
+      const cudaLaunchConfig_t cfg = resident_config<T>(ctx, &attr, c, 1, limit, ctx->stream);
+      if (cudaOccupancyMaxActiveClusters(&active[c], k_batch_resident<T>, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        active[c] = 0;
+      }
+    }
+  int cmax = RMAXC;
+  while (cmax > 0 && !active[cmax]) --cmax;
+  const int nb = w->nb;
+  std::vector<int> cl(nb, 0);
+  std::vector<ResidentInfo> info(nb);
+  auto fit = [&](int i, int c, bool whole) {
+    const i64 rows = w->off[i + 1] - w->off[i];
+    const i64 share = std::max<i64>(1, (rows + c - 1) / c);
+    const int width = std::max(1, w->width[i]), band = w->band[i];
+    if (share > RNT * RM || (share + 2 * (i64)band) * wv > 65535) return false;
+    const ResidentLayout L0(wv, (int)share, band, width, 0);
+    if (L0.end + 64 > limit) return false;
+    const i64 per = (i64)width * wv + (width + 1) / 2 * 4;
+    const i64 cap = std::min<i64>(share, (i64)(limit - L0.end - 64) / per);
+    if (whole ? cap < share : 4 * cap < share) return false;
+    cl[i] = c;
+    info[i] = ResidentInfo{width, band, (int)cap, (int)share};
+    return true;
+  };
+  i64 ctas = 0;
+  for (int i = 0; i < nb; ++i) {
+    const double rows = (double)(w->off[i + 1] - w->off[i]);
+    if (w->width[i] > RMAX_WIDTH || w->width[i] > 2.0 * w->nnz[i] / std::max(rows, 1.0) + 4.0) continue;
+    for (int c = 1; c <= cmax && !cl[i]; ++c) fit(i, c, true);
+    if (cl[i]) {  // a larger cluster of which as many run (67 -> 62 ms for the 256)
+      int c = cl[i];
+      while (c < cmax && active[c + 1] == active[cl[i]]) ++c;
+      fit(i, c, true);
+    } else {
+      fit(i, cmax, false);
+    }
+    ctas += cl[i];
+  }
+  // A few instances leave SMs idle: spread them over larger clusters while a
+  // thread keeps a row (one 64^2 instance, FP64: 3.6 us per iteration on 8 SMs,
+  // 4.9 on one).
+  for (bool grown = true; grown && 2 * ctas <= ctx->num_sms;) {
+    grown = false;
+    for (int i = 0; i < nb; ++i) {
+      const int c = cl[i], to = std::min(2 * c, cmax);
+      if (to > c && w->off[i + 1] - w->off[i] >= (i64)to * RNT && fit(i, to, true)) {
+        ctas += to - c;
+        grown = true;
+      }
+    }
+  }
+  std::vector<int> lists;
+  auto& classes = w->classes[k];
+  classes.clear();
+  for (int c = RMAXC; c > 0; --c) {
+    ResidentClass rc;
+    rc.cluster = c;
+    rc.first = (int)lists.size();
+    for (int i : by_cost)
+      if (cl[i] == c) {
+        const ResidentInfo& in = info[i];
+        rc.smem = std::max(rc.smem, ResidentLayout(wv, in.share, in.band, in.width, in.cap).end);
+        lists.push_back(i);
+      }
+    rc.count = (int)lists.size() - rc.first;
+    // Clusters are placed kernel by kernel: while clusters of 16 wait for one of
+    // the 7 places there are, the SMs beside them idle unless the grid ends at 7.
+    rc.clusters = 2 * c > cmax ? std::min(rc.count, active[c]) : rc.count;
+    if (rc.count) classes.push_back(rc);
+  }
+  w->nqueue[k] = nb - (int)lists.size();
+  for (int i : by_cost)
+    if (!cl[i]) lists.push_back(i);
+  w->turns.alloc(RMAXC + 1);
+  upload(ctx, w->lists[k], lists.data(), nb);
+  upload(ctx, w->info[k], info.data(), nb);
+  CUDA_CHECK(cudaStreamSynchronize(ctx->stream));  // host temporaries
+}
+
+template <class T>
+void launch_resident(fcu_ctx ctx, BatchWorkspace* w, const ResidentClass& rc, const BatchArgs& a,
+                     cudaStream_t stream) {
+  const int k = sizeof(T) == 4 ? 1 : 0;
+  resident_limit<T>(ctx);
+  cudaLaunchAttribute attr;
+  const cudaLaunchConfig_t cfg = resident_config<T>(ctx, &attr, rc.cluster, rc.clusters, rc.smem, stream);
+  CUDA_CHECK(cudaLaunchKernelEx(&cfg, k_batch_resident<T>, a, (const int*)(w->lists[k].p + rc.first),
+                                (const ResidentInfo*)w->info[k].p, rc.count, w->turns.p + rc.cluster));
+}
+
+// Every launch of the batch: the resident classes, largest clusters first, and
+// the queue kernel, side by side on branches of the context's stream.
+void launch_all(fcu_matrix m, BatchWorkspace* w, bool mixed, double tol, i64 max_iter) {
+  fcu_ctx ctx = m->ctx;
+  const int k = mixed ? 1 : 0;
+  const BatchArgs a = make_args(m, w, mixed, tol, max_iter);
+  const size_t branches = w->classes[k].size() + (w->nqueue[k] ? 1 : 0);
+  while (w->side.size() + 1 < branches) {
+    cudaStream_t t;
+    CUDA_CHECK(cudaStreamCreateWithFlags(&t, cudaStreamNonBlocking));
+    w->side.push_back(t);
+  }
+  while (w->joins.size() < branches) {
+    cudaEvent_t e;
+    CUDA_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    w->joins.push_back(e);
+  }
+  CUDA_CHECK(cudaMemsetAsync(w->turns.p, 0, (RMAXC + 1) * sizeof(int), ctx->stream));
+  if (branches > 1) CUDA_CHECK(cudaEventRecord(w->joins[branches - 1], ctx->stream));  // fork
+  for (size_t b = 0; b < branches; ++b) {
+    cudaStream_t st = b == 0 ? ctx->stream : w->side[b - 1];
+    if (b > 0) CUDA_CHECK(cudaStreamWaitEvent(st, w->joins[branches - 1], 0));
+    if (b < w->classes[k].size()) {
+      if (mixed) launch_resident<float>(ctx, w, w->classes[k][b], a, st);
+      else launch_resident<double>(ctx, w, w->classes[k][b], a, st);
+    } else {
+      const BatchConfig c = w->cfg[k];
+      BatchKernel kern = pick_kernel(mixed, c, w->nqueue[k]);
+      const int grid = batch_grid(ctx, kern, c, w->nqueue[k]);
+      if (grid <= 0) fail(FCU_ERR_UNSUPPORTED, "batched PCG configuration does not fit this device");
+      launch_batch(st, w, kern, c, grid, a);
+    }
+  }
+  for (size_t b = 1; b < branches; ++b) {  // join
+    CUDA_CHECK(cudaEventRecord(w->joins[b - 1], w->side[b - 1]));
+    CUDA_CHECK(cudaStreamWaitEvent(ctx->stream, w->joins[b - 1], 0));
+  }
 }
 
 }  // namespace
@@ -634,29 +1154,29 @@ int batch_pcg_impl(fcu_matrix m, i64 nb, const i64* offsets_host, const double* 
     w->nb = (int)nb;
     w->off.assign(offsets_host, offsets_host + nb + 1);
     upload(ctx, w->off_d, w->off.data(), nb + 1);
-    DBuf<int> bad;
-    bad.alloc(1);
-    CUDA_CHECK(cudaMemsetAsync(bad.p, 0, sizeof(int), ctx->stream));
-    k_batch_check<<<(unsigned)nb, 256, 0, ctx->stream>>>(m->row_ptr, m->col_idx, w->off_d.p, (int)nb, bad.p);
+    DBuf<int> chk;  // [4 per instance: entries, longest row, bandwidth, -][a column outside its block]
+    chk.alloc(4 * nb + 1);
+    CUDA_CHECK(cudaMemsetAsync(chk.p, 0, chk.bytes(), ctx->stream));
+    const unsigned per = (unsigned)std::max<i64>(1, std::min<i64>(64, 4 * ctx->num_sms / nb));
+    k_batch_check<<<dim3((unsigned)nb, per), 256, 0, ctx->stream>>>(m->row_ptr, m->col_idx, w->off_d.p, (int)nb,
+                                                                   chk.p + 4 * nb, chk.p);
     LAUNCH_CHECK(ctx);
-    int hbad = 0;
-    download(ctx, &hbad, bad.p, 1);
-    if (hbad) fail(FCU_ERR_BAD_ARG, "matrix is not block diagonal over the given offsets");
-    // queue order: estimated cost (stored entries x sqrt(rows), the 2D
-    // iteration growth), largest first
-    std::vector<int> hrp(nb + 1);
-    std::vector<int> rpv(m->n + 1);
-    download(ctx, rpv.data(), m->row_ptr, m->n + 1);
-    std::vector<double> cost(nb);
-    for (i64 i = 0; i < nb; ++i) {
-      const double rows = (double)(offsets_host[i + 1] - offsets_host[i]);
-      const double nnz = (double)(rpv[offsets_host[i + 1]] - rpv[offsets_host[i]]);
-      cost[i] = (nnz + rows) * std::sqrt(std::max(rows, 1.0));
+    std::vector<int> hc(4 * nb + 1);
+    download(ctx, hc.data(), chk.p, hc.size());
+    CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
+    if (hc[4 * nb]) {
+      delete w;  // not to be taken for a checked layout by the next call
+      w = nullptr;
+      fail(FCU_ERR_BAD_ARG, "matrix is not block diagonal over the given offsets");
     }
-    std::vector<int> ord(nb);
-    for (i64 i = 0; i < nb; ++i) ord[i] = (int)i;
-    std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) { return cost[a] > cost[b]; });
-    upload(ctx, w->order, ord.data(), nb);
+    w->nnz.resize(nb);
+    w->width.resize(nb);
+    w->band.resize(nb);
+    for (i64 i = 0; i < nb; ++i) {
+      w->nnz[i] = hc[4 * i];
+      w->width[i] = hc[4 * i + 1];
+      w->band[i] = hc[4 * i + 2];
+    }
     const i64 n = m->n;
     w->b.alloc(n);
     w->x.alloc(n);
@@ -670,18 +1190,6 @@ int batch_pcg_impl(fcu_matrix m, i64 nb, const i64* offsets_host, const double* 
     w->status.alloc(nb);
   }
   const i64 n = m->n;
-  if (mixed && !w->z32.p) {
-    w->z32.alloc(n);
-    w->p32.alloc(n);
-    w->q32.alloc(n);
-    w->ap32.alloc(n);
-  }
-  if (!mixed && !w->z64.p) {
-    w->z64.alloc(n);
-    w->p64.alloc(n);
-    w->q64.alloc(n);
-    w->ap64.alloc(n);
-  }
   cudaEvent_t e0, e1;
   CUDA_CHECK(cudaEventCreate(&e0));
   CUDA_CHECK(cudaEventCreate(&e1));
@@ -692,44 +1200,68 @@ int batch_pcg_impl(fcu_matrix m, i64 nb, const i64* offsets_host, const double* 
   CUDA_CHECK(cudaMemcpyAsync(w->b.p, b_dev, n * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
   const int k = mixed ? 1 : 0;
   if (!w->tuned[k]) {
-    if (fixed_shape) {
+    // largest first by estimated cost: stored entries x sqrt(rows), the 2D
+    // iteration growth
+    std::vector<double> cost(nb);
+    std::vector<int> ord(nb);
+    for (i64 i = 0; i < nb; ++i) {
+      const double rows = (double)(offsets_host[i + 1] - offsets_host[i]);
+      cost[i] = ((double)w->nnz[i] + rows) * std::sqrt(std::max(rows, 1.0));
+      ord[i] = (int)i;
+    }
+    std::stable_sort(ord.begin(), ord.end(), [&](int p, int q) { return cost[p] > cost[q]; });
+    if (mixed) plan_resident<float>(m, w, ord);
+    else plan_resident<double>(m, w, ord);
+    if (w->nqueue[k] && mixed) {
+      w->z32.alloc(n);
+      w->p32.alloc(n);
+      w->q32.alloc(n);
+      w->ap32.alloc(n);
+    } else if (w->nqueue[k]) {
+      w->z64.alloc(n);
+      w->p64.alloc(n);
+      w->q64.alloc(n);
+      w->ap64.alloc(n);
+    }
+    if (w->nqueue[k] == 0) {
+      w->cfg[k].vpr = 1;
+      w->cfg[k].threads = RNT;
+      w->cfg[k].cluster = w->classes[k][0].cluster;
+    } else if (fixed_shape) {
       w->cfg[k].vpr = fixed_shape[0];
       w->cfg[k].threads = fixed_shape[1];
       w->cfg[k].cluster = fixed_shape[2];
-      if (!pick_kernel(mixed, w->cfg[k], w->nb)) fail(FCU_ERR_BAD_ARG, "no batched PCG kernel of that shape");
+      if (!pick_kernel(mixed, w->cfg[k], w->nqueue[k])) fail(FCU_ERR_BAD_ARG, "no batched PCG kernel of that shape");
     } else {
       w->cfg[k] = autotune(m, w, mixed, tol);
     }
     w->tuned[k] = true;
   }
-  const BatchConfig c = w->cfg[k];
-  BatchKernel kern = pick_kernel(mixed, c, w->nb);
-  const int key = (c.vpr * 4096 + c.threads) * 16 + c.cluster;
-  if (!w->graph[k] || w->graph_key[k] != key || w->tol_g[k] != tol || w->iters_g[k] != max_iter) {
-    if (w->graph[k]) {
-      cudaGraphExecDestroy(w->graph[k]);
-      w->graph[k] = nullptr;
+  if (w->classes[k].size() + (w->nqueue[k] ? 1 : 0) == 1 && !w->nqueue[k]) {
+    launch_all(m, w, mixed, tol, max_iter);  // one launch: nothing to capture
+  } else {
+    if (!w->graph[k] || w->tol_g[k] != tol || w->iters_g[k] != max_iter) {
+      if (w->graph[k]) {
+        cudaGraphExecDestroy(w->graph[k]);
+        w->graph[k] = nullptr;
+      }
+      cudaGraph_t g;
+      CUDA_CHECK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
+      try {
+        launch_all(m, w, mixed, tol, max_iter);
+      } catch (...) {
+        cudaStreamEndCapture(ctx->stream, &g);
+        throw;
+      }
+      CUDA_CHECK(cudaStreamEndCapture(ctx->stream, &g));
+      CUDA_CHECK(cudaGraphInstantiate(&w->graph[k], g, 0));
+      cudaGraphDestroy(g);
+      w->tol_g[k] = tol;
+      w->iters_g[k] = max_iter;
     }
-    const BatchArgs a = make_args(m, w, mixed, tol, max_iter);
-    cudaGraph_t g;
-    CUDA_CHECK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-    const int grid = batch_grid(ctx, kern, c, w->nb);
-    if (grid <= 0) fail(FCU_ERR_UNSUPPORTED, "batched PCG configuration does not fit this device");
-    try {
-      launch_batch(ctx, w, kern, c, grid, a);
-    } catch (...) {
-      cudaStreamEndCapture(ctx->stream, &g);
-      throw;
-    }
-    CUDA_CHECK(cudaStreamEndCapture(ctx->stream, &g));
-    CUDA_CHECK(cudaGraphInstantiate(&w->graph[k], g, 0));
-    cudaGraphDestroy(g);
-    w->graph_key[k] = key;
-    w->tol_g[k] = tol;
-    w->iters_g[k] = max_iter;
+    CUDA_CHECK(cudaGraphLaunch(w->graph[k], ctx->stream));
   }
-  CUDA_CHECK(cudaGraphLaunch(w->graph[k], ctx->stream));
-  ctx->launches += 1;
+  ctx->launches += (i64)w->classes[k].size() + (w->nqueue[k] ? 1 : 0);
   CUDA_CHECK(cudaMemcpyAsync(x_dev, w->x.p, n * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
   CUDA_CHECK(cudaEventRecord(e1, ctx->stream));
   CUDA_CHECK(cudaEventSynchronize(e1));

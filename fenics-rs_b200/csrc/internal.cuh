@@ -104,6 +104,9 @@ struct fcu_ctx_s {
   // stored blocks, longest row, precision): a later matrix of the same shape
   // (a new solve on the same mesh) takes them without timing candidates.
   std::map<std::array<i64, 5>, std::array<int, 2>> spmv_tune;
+  // Clusters of 1..16 CTAs of the resident batched PCG that the device runs at
+  // a time (FP64, FP32), filled by the first batch.
+  std::array<int, 17> batch_clusters[2] = {};
   // Pinned solver state records of released matrices, reused by later ones
   // (pinned allocation and release are slow and synchronising), freed with
   // the context.

@@ -234,9 +234,12 @@ int fcu_solve_csr_cg(fcu_ctx ctx, int64_t n, const uint32_t* row_ptr, const uint
  * offsets[0] = 0, offsets[nb] = n) - e.g. assembled on a mesh that
  * concatenates the instances' meshes. Every block is solved from x0 = 0 with
  * its own alpha, beta and stopping test ||r_i|| / ||b_i|| < tol, as
- * fcu_pcg would solve it alone (precision FCU_FP64 or FCU_MIXED), in one
- * persistent launch (captured in a CUDA graph, replayed on later calls):
- * each instance is taken by a cluster of 1-8 CTAs, largest instances first.
+ * fcu_pcg would solve it alone (precision FCU_FP64 or FCU_MIXED): each
+ * instance is held on chip by a thread-block cluster of 1-16 CTAs for the whole
+ * of its solve, one launch per cluster size, side by side (several launches are
+ * captured in a CUDA graph and replayed on later calls). Instances too large or
+ * with rows too long for that stream their data through a queue of clusters of
+ * 1-8 CTAs. Largest instances first.
  * Per-instance iterations, relative residuals and statuses go to the
  * optional host arrays (nb each). Returns FCU_OK when every instance
  * converged, else the first failing status. info: max iterations, total
@@ -245,8 +248,9 @@ int fcu_batch_pcg(fcu_ctx ctx, fcu_matrix m, int64_t nb, const int64_t* offsets,
                   double tol, int64_t max_iter, int precision, int64_t* iterations, double* rel_residual,
                   int* status, fcu_solve_info* info);
 /* Lanes per row, threads per CTA and CTAs per instance (thread-block
- * cluster) that the batched solver's tuning chose for m and `precision`
- * (all 0 before its first solve). */
+ * cluster) of the batched solver for m and `precision` (all 0 before its first
+ * solve): those of the queue if any instance takes it, else those of the
+ * largest cluster. */
 int fcu_batch_config(fcu_matrix m, int precision, int* lanes_per_row, int* threads_per_cta,
                      int* ctas_per_cluster);
 
