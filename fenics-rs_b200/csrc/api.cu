@@ -35,7 +35,7 @@ void time_pcg_impl(fcu_matrix m, int precision, i64 iters, int reps, size_t flus
 void check_wait_limits_impl(fcu_ctx ctx, unsigned limit, int* results_host);
 int batch_pcg_impl(fcu_matrix m, i64 nb, const i64* offsets_host, const double* b_dev, double* x_dev, double tol,
                    i64 max_iter, int precision, i64* iters_host, double* relres_host, int* status_host,
-                   fcu_solve_info* info, const int* fixed_shape = nullptr);
+                   fcu_solve_info* info, bool on_chip_only);
 void batch_config(fcu_matrix m, int precision, int* vpr, int* threads, int* cluster);
 void element_stresses_impl(fcu_space s, double lam, double mu, const double* u_dev, double* stress, double* strain,
                            double* vm, double* trace);
@@ -1242,7 +1242,7 @@ int fcu_batch_pcg(fcu_ctx ctx, fcu_matrix m, int64_t nb, const int64_t* offsets,
     DevIn<double> bd(ctx, b, m->n);
     DevOut<double> xo(x, m->n);
     st = batch_pcg_impl(m, nb, offs.data(), bd.p, xo.p, tol, max_iter, precision, iterations, rel_residual, status,
-                        info);
+                        info, false);
     xo.finish(ctx);
     sync(ctx);
   });

@@ -20,11 +20,12 @@
 // later solves replay. The streaming form's lanes per row, threads per CTA and
 // CTAs per cluster are picked by timing the candidates on its instances (first
 // solve of a matrix and precision), unless FCU_BATCH_VPR / FCU_BATCH_THREADS /
-// FCU_BATCH_CLUSTER fix them; a single system (the small-system path of the
-// PCG) takes a shape fixed by rule.
+// FCU_BATCH_CLUSTER fix them. A single system (the small-system path of the PCG)
+// is taken if all of it fits on chip.
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -801,7 +802,8 @@ struct BatchWorkspace {
   std::vector<cudaStream_t> side;     // branches of the captured launch
   std::vector<cudaEvent_t> joins;
   BatchConfig cfg[2];
-  bool tuned[2] = {false, false};
+  bool planned[2] = {false, false}, tuned[2] = {false, false};
+  bool on_chip[2] = {false, false};   // every instance is resident, with all of its rows
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
   double tol_g[2] = {0.0, 0.0};
   i64 iters_g[2] = {0, 0};
@@ -1070,6 +1072,8 @@ void plan_resident(fcu_matrix m, BatchWorkspace* w, const std::vector<int>& by_c
     if (rc.count) classes.push_back(rc);
   }
   w->nqueue[k] = nb - (int)lists.size();
+  w->on_chip[k] = w->nqueue[k] == 0;
+  for (int i = 0; i < nb; ++i) w->on_chip[k] = w->on_chip[k] && info[i].cap >= info[i].share;
   for (int i : by_cost)
     if (!cl[i]) lists.push_back(i);
   w->turns.alloc(RMAXC + 1);
@@ -1134,7 +1138,7 @@ void launch_all(fcu_matrix m, BatchWorkspace* w, bool mixed, double tol, i64 max
 // buffers handled by the caller (api.cu) through staging.
 int batch_pcg_impl(fcu_matrix m, i64 nb, const i64* offsets_host, const double* b_dev, double* x_dev, double tol,
                    i64 max_iter, int precision, i64* iters_host, double* relres_host, int* status_host,
-                   fcu_solve_info* info, const int* fixed_shape) {
+                   fcu_solve_info* info, bool on_chip_only) {
   fcu_ctx ctx = m->ctx;
   const bool mixed = precision == FCU_MIXED;
   if (m->bs != 1) fail(FCU_ERR_UNSUPPORTED, "batched PCG takes scalar (CSR) matrices");
@@ -1146,11 +1150,12 @@ int batch_pcg_impl(fcu_matrix m, i64 nb, const i64* offsets_host, const double* 
     if (offsets_host[i + 1] < offsets_host[i]) fail(FCU_ERR_BAD_ARG, "offsets must not decrease");
   if (max_iter < 0) fail(FCU_ERR_BAD_ARG, "max_iter must be non-negative");
 
-  BatchWorkspace*& w = m->bws;
-  const bool same = w && w->nb == nb && std::equal(w->off.begin(), w->off.end(), offsets_host);
+  const bool same =
+      m->bws && m->bws->nb == nb && std::equal(m->bws->off.begin(), m->bws->off.end(), offsets_host);
   if (!same) {
-    delete w;
-    w = new BatchWorkspace();
+    delete m->bws;
+    m->bws = nullptr;
+    std::unique_ptr<BatchWorkspace> w(new BatchWorkspace());  // kept once it is complete
     w->nb = (int)nb;
     w->off.assign(offsets_host, offsets_host + nb + 1);
     upload(ctx, w->off_d, w->off.data(), nb + 1);
@@ -1164,11 +1169,7 @@ int batch_pcg_impl(fcu_matrix m, i64 nb, const i64* offsets_host, const double* 
     std::vector<int> hc(4 * nb + 1);
     download(ctx, hc.data(), chk.p, hc.size());
     CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
-    if (hc[4 * nb]) {
-      delete w;  // not to be taken for a checked layout by the next call
-      w = nullptr;
-      fail(FCU_ERR_BAD_ARG, "matrix is not block diagonal over the given offsets");
-    }
+    if (hc[4 * nb]) fail(FCU_ERR_BAD_ARG, "matrix is not block diagonal over the given offsets");
     w->nnz.resize(nb);
     w->width.resize(nb);
     w->band.resize(nb);
@@ -1188,18 +1189,11 @@ int batch_pcg_impl(fcu_matrix m, i64 nb, const i64* offsets_host, const double* 
     w->relres.alloc(nb);
     w->resid.alloc(nb);
     w->status.alloc(nb);
+    m->bws = w.release();
   }
-  const i64 n = m->n;
-  cudaEvent_t e0, e1;
-  CUDA_CHECK(cudaEventCreate(&e0));
-  CUDA_CHECK(cudaEventCreate(&e1));
-  CUDA_CHECK(cudaEventRecord(e0, ctx->stream));
-  k_batch_invd<<<grid_for(n, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(m->diag_pos, m->val64.p, n, w->invd.p);
-  LAUNCH_CHECK(ctx);
-  if (mixed) build_rowsum32(m);
-  CUDA_CHECK(cudaMemcpyAsync(w->b.p, b_dev, n * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
+  BatchWorkspace* const w = m->bws;
   const int k = mixed ? 1 : 0;
-  if (!w->tuned[k]) {
+  if (!w->planned[k]) {
     // largest first by estimated cost: stored entries x sqrt(rows), the 2D
     // iteration growth
     std::vector<double> cost(nb);
@@ -1212,6 +1206,19 @@ int batch_pcg_impl(fcu_matrix m, i64 nb, const i64* offsets_host, const double* 
     std::stable_sort(ord.begin(), ord.end(), [&](int p, int q) { return cost[p] > cost[q]; });
     if (mixed) plan_resident<float>(m, w, ord);
     else plan_resident<double>(m, w, ord);
+    w->planned[k] = true;
+  }
+  if (on_chip_only && !w->on_chip[k]) return BATCH_NOT_ON_CHIP;
+  const i64 n = m->n;
+  cudaEvent_t e0, e1;
+  CUDA_CHECK(cudaEventCreate(&e0));
+  CUDA_CHECK(cudaEventCreate(&e1));
+  CUDA_CHECK(cudaEventRecord(e0, ctx->stream));
+  k_batch_invd<<<grid_for(n, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(m->diag_pos, m->val64.p, n, w->invd.p);
+  LAUNCH_CHECK(ctx);
+  if (mixed) build_rowsum32(m);
+  CUDA_CHECK(cudaMemcpyAsync(w->b.p, b_dev, n * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
+  if (!w->tuned[k]) {
     if (w->nqueue[k] && mixed) {
       w->z32.alloc(n);
       w->p32.alloc(n);
@@ -1227,11 +1234,6 @@ int batch_pcg_impl(fcu_matrix m, i64 nb, const i64* offsets_host, const double* 
       w->cfg[k].vpr = 1;
       w->cfg[k].threads = RNT;
       w->cfg[k].cluster = w->classes[k][0].cluster;
-    } else if (fixed_shape) {
-      w->cfg[k].vpr = fixed_shape[0];
-      w->cfg[k].threads = fixed_shape[1];
-      w->cfg[k].cluster = fixed_shape[2];
-      if (!pick_kernel(mixed, w->cfg[k], w->nqueue[k])) fail(FCU_ERR_BAD_ARG, "no batched PCG kernel of that shape");
     } else {
       w->cfg[k] = autotune(m, w, mixed, tol);
     }

@@ -117,6 +117,9 @@ struct fcu_ctx_s {
   }
 };
 
+// Answer of the batched PCG when asked for systems that are held on chip only.
+constexpr int BATCH_NOT_ON_CHIP = -1;
+
 struct fcu_mesh_s {
   int refs = 1;
   fcu_ctx ctx = nullptr;

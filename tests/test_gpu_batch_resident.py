@@ -81,3 +81,23 @@ def test_offsets_refused_twice_then_accepted(fcu, ctx):
     x, _, _, st, _ = M.batch_pcg(offs, b, tol=1e-12)
     assert np.all(st == 0) and np.linalg.norm(b - A @ x) < 3e-12 * np.linalg.norm(b)
     M.close()
+
+
+@pytest.mark.parametrize("n,pattern", [
+    (60000, lambda n: (1, 250)),                 # the largest that is tried on chip
+    (60001, lambda n: (1, 250)),
+    (30000, lambda n: tuple(range(1, 8))),       # FP64 does not fit, FP32 does
+    (30000, lambda n: (1, 14999)),               # fits but for its bandwidth
+    (5000, lambda n: tuple(range(1, 17))),       # rows too long
+])
+def test_single_systems_on_both_sides_of_the_on_chip_limit(fcu, ctx, n, pattern):
+    rng = np.random.default_rng(n)
+    A, M, _ = _batch(fcu, ctx, [_block(n, pattern(n), rng)])
+    b = rng.standard_normal(n)
+    for prec in (fcu.FCU_FP64, fcu.FCU_MIXED, fcu.FCU_FP64):
+        x, info = M.pcg(b, tol=1e-12, max_iter=2000, precision=prec)
+        assert info.status == 0 and np.linalg.norm(b - A @ x) < 3e-12 * np.linalg.norm(b)
+    # a solve of one system between two batches on the same matrix
+    y, _, _, st, _ = M.batch_pcg([0, n], b, tol=1e-12, max_iter=2000)
+    assert np.all(st == 0) and np.linalg.norm(b - A @ y) < 3e-12 * np.linalg.norm(b)
+    M.close()
