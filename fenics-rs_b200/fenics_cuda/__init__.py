@@ -384,12 +384,10 @@ class FunctionSpace:
             pass
 
     def boundary_dofs(self) -> np.ndarray:
-        n = C.c_int64(0)
-        _check(self.ctx, _L().fcu_space_boundary_dofs(self.ctx.h, self.h, None, C.byref(n)))
-        out = np.empty(n.value, np.int64)
-        if n.value:
-            _check(self.ctx, _L().fcu_space_boundary_dofs(self.ctx.h, self.h, out.ctypes.data, C.byref(n)))
-        return out
+        n = C.c_int64(self.ndofs)
+        out = np.empty(self.ndofs, np.int64)  # room for every dof: one call, not one to count and one to fill
+        _check(self.ctx, _L().fcu_space_boundary_dofs(self.ctx.h, self.h, out.ctypes.data, C.byref(n)))
+        return out[:n.value].copy()
 
     def p2_dofmap(self):
         cd = np.empty((self.mesh.nc, 10), np.int64)
@@ -769,12 +767,10 @@ def boundary_dofs_3d(mesh: Mesh, ctx: Context | None = None) -> np.ndarray:
 def _boundary_dofs(mesh: Mesh, ctx):
     ctx = ctx or default_context()
     h = mesh.handle(ctx)
-    n = C.c_int64(0)
-    _check(ctx, _L().fcu_boundary_dofs(ctx.h, h, None, C.byref(n)))
-    out = np.empty(n.value, np.int64)
-    if n.value:
-        _check(ctx, _L().fcu_boundary_dofs(ctx.h, h, out.ctypes.data, C.byref(n)))
-    return out
+    n = C.c_int64(mesh.nv)
+    out = np.empty(mesh.nv, np.int64)
+    _check(ctx, _L().fcu_boundary_dofs(ctx.h, h, out.ctypes.data, C.byref(n)))
+    return out[:n.value].copy()
 
 
 @dataclass
