@@ -14,7 +14,7 @@
 //     row evaluates each of the row's cells' element rows into shared memory
 //     (the row's "contributions", ascending cell id), then each lane sums the
 //     entries of its slot in ascending cell order;
-//   * P2: per-cell metric records, then three rows per warp, a lane per local
+//   * P2: per-cell Gram records, then three rows per warp, a lane per local
 //     column, adding each contribution's entry into the row's shared-memory
 //     accumulators (k_assemble_p2_rows);
 //   * vector-P1 elasticity and mass: per-cell records (gradients and scale,
@@ -22,6 +22,8 @@
 //     the block's cell list, the diagonal block from the row (k_elast_rows,
 //     k_mass_rows_vec).
 // Rows are written with coalesced stores in every form.
+
+#include <type_traits>
 
 #include "internal.cuh"
 
@@ -152,46 +154,129 @@ __global__ void k_p2_metric_records(const int* __restrict__ cn, const double* __
   }
 }
 
+// Gram record of a P2 cell: grad l_i . grad l_j of the barycentric coordinates
+// for i <= j (00, 01, 02, 03, 11, 12, 13, 22, 23, 33), times kappa |det J| / 30.
+constexpr int P2_GRAM = 10;
+
+__global__ void k_p2_gram_records(const int* __restrict__ cn, const double* __restrict__ X,
+                                  const double* __restrict__ coef, i64 nc, double* __restrict__ gram) {
+  for (i64 c = blockIdx.x * (i64)blockDim.x + threadIdx.x; c < nc; c += (i64)gridDim.x * blockDim.x) {
+    int v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = cn[c * 10 + i];
+    const Geo3 g = tet_geometry(X, v);
+    const double s = fabs(g.det) * (coef ? coef[c] : 1.0) * (1.0 / 30.0);
+    double gr[4][3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      gr[1][r] = g.G[r][0];
+      gr[2][r] = g.G[r][1];
+      gr[3][r] = g.G[r][2];
+      gr[0][r] = -g.G[r][0] - g.G[r][1] - g.G[r][2];
+    }
+    double G[P2_GRAM];
+    int m = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = i; j < 4; ++j) G[m++] = (gr[i][0] * gr[j][0] + gr[i][1] * gr[j][1] + gr[i][2] * gr[j][2]) * s;
+    double2* o = reinterpret_cast<double2*>(gram + c * P2_GRAM);
+#pragma unroll
+    for (int q = 0; q < P2_GRAM / 2; ++q) o[q] = make_double2(G[2 * q], G[2 * q + 1]);
+  }
+}
+
+// Entry (a, b) of the P2 element stiffness as four Gram entries with small whole
+// coefficients: with w(i, j) = 3 if i == j else -1 and d(i, j) = 8 if i == j else
+// 4, vertices i, j give w(i, j) G_ij; vertex i and edge jk w(i, j) G_ik +
+// w(i, k) G_ij; edges ij and kl d(i, k) G_jl + d(i, l) G_jk + d(j, k) G_il +
+// d(j, l) G_ik (exact integrals of the products of linear gradients; the
+// degree-2 rule integrates them exactly too). x: per term the two byte
+// selectors of p2_coef, y: the Gram entry's number; a byte each.
+struct P2Terms {
+  unsigned x[100], y[100];  // [10 a + b]
+};
+constexpr P2Terms make_p2_terms() {
+  P2Terms T{};
+  const int E0[10] = {0, 1, 2, 3, 0, 1, 0, 0, 1, 2}, E1[10] = {0, 1, 2, 3, 1, 2, 2, 3, 3, 3};
+  for (int a = 0; a < 10; ++a)
+    for (int b = 0; b < 10; ++b) {
+      // terms: coefficient w or d of (ci, cj), Gram entry (gi, gj)
+      int n = 0, ci[4] = {}, cj[4] = {}, gi[4] = {}, gj[4] = {};
+      const bool edges = a >= 4 && b >= 4;
+      if (a < 4 && b < 4) {
+        n = 1;
+        ci[0] = gi[0] = a;
+        cj[0] = gj[0] = b;
+      } else if (!edges) {
+        const int i = a < 4 ? a : b, e = a < 4 ? b : a;
+        n = 2;
+        for (int q = 0; q < 2; ++q) {
+          ci[q] = gi[q] = i;
+          cj[q] = q ? E1[e] : E0[e];
+          gj[q] = q ? E0[e] : E1[e];
+        }
+      } else {
+        n = 4;
+        for (int q = 0; q < 4; ++q) {
+          ci[q] = q < 2 ? E0[a] : E1[a];
+          gi[q] = q < 2 ? E1[a] : E0[a];
+          cj[q] = q % 2 ? E1[b] : E0[b];
+          gj[q] = q % 2 ? E0[b] : E1[b];
+        }
+      }
+      for (int q = 0; q < n; ++q) {
+        const unsigned coef = edges ? (ci[q] == cj[q] ? 0x54u : 0x53u) : (ci[q] == cj[q] ? 0x51u : 0x62u);
+        const int lo = gi[q] < gj[q] ? gi[q] : gj[q], hi = gi[q] < gj[q] ? gj[q] : gi[q];
+        T.x[10 * a + b] |= coef << (8 * q);
+        T.y[10 * a + b] |= (unsigned)(4 * lo - lo * (lo - 1) / 2 + hi - lo) << (8 * q);
+      }
+    }
+  return T;
+}
+__constant__ P2Terms c_p2_terms = make_p2_terms();
+
+// Selectors to the coefficient: 0x51 3, 0x62 -1, 0x53 4, 0x54 8, 0x00 0 (the
+// upper two bytes of the double, out of a table of eight bytes).
+__device__ __forceinline__ double p2_coef(unsigned x, int term) {
+  const unsigned sel = (term == 0 ? x << 8 : x >> (8 * (term - 1))) & 0xff00u;
+  return __hiloint2double((int)__byte_perm(0x10F00800u, 0x00BF4020u, sel), 0);
+}
+
 // P2 stiffness, three rows per warp (the kernel fcu_assemble_stiffness runs on
 // P2 spaces whose rows have at most 255 slots). Lanes 10g .. 10g+9 own row g
 // of the warp's three consecutive rows, lane 10g+b local column b. At each
 // step every group takes its row's next contribution (cell c with the row's
 // dof at local index a; contributions ordered by (a, c)), forms the element
-// entry K_e[a][b] = sum_m S_c[m] R[m][a][b] from the cell's metric record,
-// and adds it to the row's accumulator of slot cmap[t][b] in shared memory.
+// entry K_e[a][b] from the cell's Gram record, of which lane 10g+m holds entry
+// m, and adds it to the row's accumulator of slot cmap[t][b] in shared memory.
 // The ten columns of one cell are ten distinct dofs, so the ten lanes of a
 // group update ten distinct slots: no atomics, and every slot sums its
 // contributions in one fixed order (the values repeat bit for bit; they agree
 // with the triplet assembly's ascending-cell sums to round-off). The three
 // rows' slots are contiguous in the pattern, so the warp writes them with
-// coalesced stores. One element entry costs one metric record read (shared by
-// the group), six FMAs and one shared-memory add; no per-entry summation
-// lists are read.
+// coalesced stores.
+// Bound by the load/store unit, 92 % busy when an entry was the product of six
+// metric and six reference-tensor values: 96 bytes a lane and step. Here a lane
+// loads one Gram value a step ahead, its four operands come by shuffles and the
+// coefficients from eight bytes of a table: 64^3 cube (2.1M rows, 61M entries)
+// 1016 -> 724 us, the 16^3 one 32 -> 25 us. Still bound there (90 %; the adds into
+// the accumulators and the shuffles) and by issue (79 %). Rows of vertices, 40 %
+// of the contributions, need two terms only; many more blocks than fit at once
+// even out the rows' different lengths (8 a multiprocessor 833 us, 64 724).
 constexpr int P2W = 8;  // warps per block
 
-__device__ __forceinline__ void p2_record(const double* __restrict__ p2geo, int cc, double2& s01, double2& s23,
-                                          double2& s45) {
-  const double2* rec = reinterpret_cast<const double2*>(p2geo + (i64)(cc >> 4) * P2_GEO);
-  s01 = __ldg(rec);
-  s23 = __ldg(rec + 1);
-  s45 = __ldg(rec + 2);
-}
-
-// Each row's contributions come ordered by (local index a of the row's dof,
-// cell), so a lane keeps its six reference-tensor entries R[m][a][b] in
-// registers and reloads them from shared memory only when a changes (at most
-// four times on a vertex row, six on an edge row) instead of at every step.
 __global__ void __launch_bounds__(P2W * 32) k_assemble_p2_rows(
     const int* __restrict__ row_ptr, const int* __restrict__ contrib_ptr, const int* __restrict__ contrib_a,
-    const unsigned char* __restrict__ cmap, const double* __restrict__ p2geo, i64 nrows, int stride,
+    const unsigned char* __restrict__ cmap, const double* __restrict__ gram, i64 nrows, int stride,
     double* __restrict__ v64, float* __restrict__ v32) {
   extern __shared__ double p2sh[];
-  double* R = p2sh;  // 6 x 10 x 10
+  uint2* const terms = reinterpret_cast<uint2*>(p2sh);  // 10 x 10
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  for (int q = threadIdx.x; q < 600; q += blockDim.x) R[q] = (&c_p2_R[0][0][0])[q];
+  for (int q = threadIdx.x; q < 100; q += blockDim.x) terms[q] = make_uint2(c_p2_terms.x[q], c_p2_terms.y[q]);
   __syncthreads();
   const int g = lane / 10, b = lane - 10 * g;  // g == 3 on lanes 30 and 31
-  double* acc = p2sh + 600 + (i64)wib * 3 * stride;
+  double* acc = p2sh + 100 + (i64)wib * 3 * stride;
   double* my = acc + (g < 3 ? g : 0) * stride;
   const i64 nwarps = (i64)gridDim.x * P2W;
   for (i64 r0 = ((i64)blockIdx.x * P2W + wib) * 3; r0 < nrows; r0 += nwarps * 3) {
@@ -205,36 +290,43 @@ __global__ void __launch_bounds__(P2W * 32) k_assemble_p2_rows(
     for (int q = b; q < L; q += 10) my[q] = 0.0;
     const int steps = __reduce_max_sync(FULL, nct);
     __syncwarp();
-    int a_cur = -1;
-    double r0v = 0.0, r1v = 0.0, r2v = 0.0, r3v = 0.0, r4v = 0.0, r5v = 0.0;
-    for (int t = 0; t < steps; ++t) {
-      if (t < nct) {
-        const i64 ci = (i64)cs + t;
-        const int cc = contrib_a[ci];
-        double2 s01, s23, s45;
-        p2_record(p2geo, cc, s01, s23, s45);
-        const int sl = cmap[ci * 10 + b];
-        const int a = cc & 15;
-        if (a != a_cur) {
-          const double* Rab = R + a * 10 + b;
-          r0v = Rab[0];
-          r1v = Rab[100];
-          r2v = Rab[200];
-          r3v = Rab[300];
-          r4v = Rab[400];
-          r5v = Rab[500];
-          a_cur = a;
-        }
-        double v = s01.x * r0v;
-        v += s01.y * r1v;
-        v += s23.x * r2v;
-        v += s23.y * r3v;
-        v += s45.x * r4v;
-        v += s45.y * r5v;
-        my[sl] += v;
-      }
-      __syncwarp();
+    // lane b of a group holds the row's contribution 10 j + b
+    int chunk = b < nct ? contrib_a[cs + b] : 0, tt = 0;
+    const unsigned char* map = cmap + (i64)cs * 10 + b;
+    const unsigned lanes = 0x0A0A0A0Au * (unsigned)g;  // a group's first lane, in each byte
+    int cc1 = __shfl_sync(FULL, chunk, 10 * g), sl1 = 0;
+    double n1 = 0.0;
+    if (nct > 0) {
+      n1 = __ldg(gram + (i64)(cc1 >> 4) * P2_GRAM + b);
+      sl1 = map[0];
     }
+    auto sweep = [&](auto nterms) {
+#pragma unroll 1
+      for (int t = 0; t < steps; ++t) {
+        const uint2 d = terms[(cc1 & 15) * 10 + b];
+        const unsigned src = d.y + lanes;  // (the shuffle takes the lowest five bits)
+        const int sl = sl1;
+        const double G = n1;
+        if (++tt == 10) {
+          tt = 0;
+          chunk = t + 1 + b < nct ? contrib_a[cs + t + 1 + b] : 0;
+        }
+        cc1 = __shfl_sync(FULL, chunk, 10 * g + tt);
+        if (t + 1 < nct) {
+          n1 = __ldg(gram + (i64)(cc1 >> 4) * P2_GRAM + b);
+          sl1 = map[10 * (t + 1)];
+        }
+        double v = 0.0;
+#pragma unroll
+        for (int q = 0; q < decltype(nterms)::value; ++q)
+          v = fma(p2_coef(d.x, q), __shfl_sync(FULL, G, (int)(src >> (8 * q))), v);
+        if (t < nct) my[sl] += v;
+        __syncwarp();
+      }
+    };
+    // rows of vertices have at most two terms per entry
+    if (__all_sync(FULL, nct == 0 || (chunk & 15) < 4)) sweep(std::integral_constant<int, 2>());
+    else sweep(std::integral_constant<int, 4>());
     const i64 rend = r0 + 3 < nrows ? r0 + 3 : nrows;
     const int base = row_ptr[r0];
     const int tot = row_ptr[rend] - base;
@@ -1278,28 +1370,32 @@ void assemble_stiffness_impl(fcu_matrix m, const double* coef_dev) {
   fcu_mesh me = s->mesh;
   const int nb = assembly_blocks(ctx, s->nnodes);
   if (s->kind == FCU_SPACE_P2 || s->kind == FCU_SPACE_P2_NODES) {
-    ensure_p2_tables(ctx);
     DBuf<double> geo;
-    geo.alloc((size_t)me->nc * P2_GEO);
-    k_p2_metric_records<<<grid_for(me->nc, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(
-        s->cell_nodes.p, me->coords.p, coef_dev, me->nc, geo.p);
-    LAUNCH_CHECK(ctx);
     if (s->cmap.p && s->contrib_a.p && !p2_row_gather()) {
+      geo.alloc((size_t)me->nc * P2_GRAM);
+      k_p2_gram_records<<<grid_for(me->nc, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(
+          s->cell_nodes.p, me->coords.p, coef_dev, me->nc, geo.p);
+      LAUNCH_CHECK(ctx);
       const int stride = s->max_row | 1;  // odd, so the three rows' accumulators start in different banks
-      const size_t smem = (600 + (size_t)P2W * 3 * stride) * sizeof(double);
+      const size_t smem = (100 + (size_t)P2W * 3 * stride) * sizeof(double);
       static bool attr_set[64] = {};
       if (smem > 48 * 1024 && !attr_set[ctx->device & 63]) {
         CUDA_CHECK(cudaFuncSetAttribute(k_assemble_p2_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
         attr_set[ctx->device & 63] = true;
       }
       const i64 groups = (s->nnodes + 3 * P2W - 1) / (3 * P2W);
-      const int nbp = (int)std::max<i64>(1, std::min<i64>(groups, (i64)ctx->num_sms * 8));
+      const int nbp = (int)std::max<i64>(1, std::min<i64>(groups, (i64)ctx->num_sms * 64));
       k_assemble_p2_rows<<<nbp, P2W * 32, smem, ctx->stream>>>(s->row_ptr.p, s->contrib_ptr.p, s->contrib_a.p,
                                                                 s->cmap.p, geo.p, s->nnodes, stride, m->val64.p,
                                                                 m->val32.p);
       LAUNCH_CHECK(ctx);
       return;
     }
+    ensure_p2_tables(ctx);
+    geo.alloc((size_t)me->nc * P2_GEO);
+    k_p2_metric_records<<<grid_for(me->nc, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(
+        s->cell_nodes.p, me->coords.p, coef_dev, me->nc, geo.p);
+    LAUNCH_CHECK(ctx);
     k_assemble_scalar<10, 3, true><<<nb, WARPS * 32, 0, ctx->stream>>>(
         s->row_ptr.p, s->contrib_ptr.p, s->contrib.p, s->slot_cnt.p, s->slot_ent.p, s->cell_nodes.p, me->coords.p,
         coef_dev, geo.p, s->diag_pos.p, s->nnodes, m->val64.p, m->val32.p);
