@@ -790,9 +790,7 @@ struct BatchWorkspace {
   DBuf<double> z64, p64, q64, ap64;  // q: the second direction buffer
   DBuf<float> z32, p32, q32, ap32;
   DBuf<unsigned> counter;
-  DBuf<i64> iters, updates;
-  DBuf<double> relres, resid;
-  DBuf<int> status;
+  DBuf<i64> results;  // nb each: iterations, replacements, relative and absolute residual, status
   std::vector<int> nnz, width, band;  // per instance: entries, longest row, bandwidth
   std::vector<ResidentClass> classes[2];  // resident launches (FP64, FP32), then the instances left to the queue
   DBuf<ResidentInfo> info[2];
@@ -845,11 +843,11 @@ BatchArgs make_args(fcu_matrix m, BatchWorkspace* w, bool mixed, double tol, i64
   a.max_iter = max_iter;
   a.delta = 0.1;
   a.counter = w->counter.p;
-  a.iters = w->iters.p;
-  a.updates = w->updates.p;
-  a.relres = w->relres.p;
-  a.resid = w->resid.p;
-  a.status = w->status.p;
+  a.iters = w->results.p;
+  a.updates = w->results.p + w->nb;
+  a.relres = reinterpret_cast<double*>(w->results.p + 2 * (i64)w->nb);
+  a.resid = reinterpret_cast<double*>(w->results.p + 3 * (i64)w->nb);
+  a.status = reinterpret_cast<int*>(w->results.p + 4 * (i64)w->nb);
   return a;
 }
 
@@ -1078,8 +1076,7 @@ void plan_resident(fcu_matrix m, BatchWorkspace* w, const std::vector<int>& by_c
     if (!cl[i]) lists.push_back(i);
   w->turns.alloc(RMAXC + 1);
   upload(ctx, w->lists[k], lists.data(), nb);
-  upload(ctx, w->info[k], info.data(), nb);
-  CUDA_CHECK(cudaStreamSynchronize(ctx->stream));  // host temporaries
+  upload(ctx, w->info[k], info.data(), nb);  // (pageable copies are staged before they return)
 }
 
 template <class T>
@@ -1095,10 +1092,11 @@ void launch_resident(fcu_ctx ctx, BatchWorkspace* w, const ResidentClass& rc, co
 
 // Every launch of the batch: the resident classes, largest clusters first, and
 // the queue kernel, side by side on branches of the context's stream.
-void launch_all(fcu_matrix m, BatchWorkspace* w, bool mixed, double tol, i64 max_iter) {
+void launch_all(fcu_matrix m, BatchWorkspace* w, bool mixed, double tol, i64 max_iter, double* x) {
   fcu_ctx ctx = m->ctx;
   const int k = mixed ? 1 : 0;
-  const BatchArgs a = make_args(m, w, mixed, tol, max_iter);
+  BatchArgs a = make_args(m, w, mixed, tol, max_iter);
+  a.x = x;
   const size_t branches = w->classes[k].size() + (w->nqueue[k] ? 1 : 0);
   while (w->side.size() + 1 < branches) {
     cudaStream_t t;
@@ -1180,15 +1178,9 @@ int batch_pcg_impl(fcu_matrix m, i64 nb, const i64* offsets_host, const double* 
     }
     const i64 n = m->n;
     w->b.alloc(n);
-    w->x.alloc(n);
-    w->r.alloc(n);
     w->invd.alloc(n);
     w->counter.alloc(1);
-    w->iters.alloc(nb);
-    w->updates.alloc(nb);
-    w->relres.alloc(nb);
-    w->resid.alloc(nb);
-    w->status.alloc(nb);
+    w->results.alloc(5 * nb);
     m->bws = w.release();
   }
   BatchWorkspace* const w = m->bws;
@@ -1214,6 +1206,9 @@ int batch_pcg_impl(fcu_matrix m, i64 nb, const i64* offsets_host, const double* 
   CUDA_CHECK(cudaEventCreate(&e0));
   CUDA_CHECK(cudaEventCreate(&e1));
   CUDA_CHECK(cudaEventRecord(e0, ctx->stream));
+  const bool one_launch = w->classes[k].size() == 1 && w->nqueue[k] == 0;  // straight into x_dev
+  if (!one_launch) w->x.alloc(n);
+  if (w->nqueue[k]) w->r.alloc(n);
   k_batch_invd<<<grid_for(n, 256, ctx->num_sms * 8), 256, 0, ctx->stream>>>(m->diag_pos, m->val64.p, n, w->invd.p);
   LAUNCH_CHECK(ctx);
   if (mixed) build_rowsum32(m);
@@ -1239,8 +1234,8 @@ int batch_pcg_impl(fcu_matrix m, i64 nb, const i64* offsets_host, const double* 
     }
     w->tuned[k] = true;
   }
-  if (w->classes[k].size() + (w->nqueue[k] ? 1 : 0) == 1 && !w->nqueue[k]) {
-    launch_all(m, w, mixed, tol, max_iter);  // one launch: nothing to capture
+  if (one_launch) {
+    launch_all(m, w, mixed, tol, max_iter, x_dev);  // nothing to capture
   } else {
     if (!w->graph[k] || w->tol_g[k] != tol || w->iters_g[k] != max_iter) {
       if (w->graph[k]) {
@@ -1250,7 +1245,7 @@ int batch_pcg_impl(fcu_matrix m, i64 nb, const i64* offsets_host, const double* 
       cudaGraph_t g;
       CUDA_CHECK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
       try {
-        launch_all(m, w, mixed, tol, max_iter);
+        launch_all(m, w, mixed, tol, max_iter, w->x.p);
       } catch (...) {
         cudaStreamEndCapture(ctx->stream, &g);
         throw;
@@ -1264,24 +1259,24 @@ int batch_pcg_impl(fcu_matrix m, i64 nb, const i64* offsets_host, const double* 
     CUDA_CHECK(cudaGraphLaunch(w->graph[k], ctx->stream));
   }
   ctx->launches += (i64)w->classes[k].size() + (w->nqueue[k] ? 1 : 0);
-  CUDA_CHECK(cudaMemcpyAsync(x_dev, w->x.p, n * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
+  if (!one_launch)
+    CUDA_CHECK(cudaMemcpyAsync(x_dev, w->x.p, n * sizeof(double), cudaMemcpyDeviceToDevice, ctx->stream));
   CUDA_CHECK(cudaEventRecord(e1, ctx->stream));
-  CUDA_CHECK(cudaEventSynchronize(e1));
+  std::vector<i64> results(5 * nb);
+  download(ctx, results.data(), w->results.p, results.size());
+  CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
   float ms = 0.f;
   CUDA_CHECK(cudaEventElapsedTime(&ms, e0, e1));
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  std::vector<i64> it(nb), up(nb);
-  std::vector<double> rel(nb), res(nb);
-  std::vector<int> st(nb);
-  download(ctx, it.data(), w->iters.p, nb);
-  download(ctx, up.data(), w->updates.p, nb);
-  download(ctx, rel.data(), w->relres.p, nb);
-  download(ctx, res.data(), w->resid.p, nb);
-  download(ctx, st.data(), w->status.p, nb);
-  if (iters_host) std::copy(it.begin(), it.end(), iters_host);
-  if (relres_host) std::copy(rel.begin(), rel.end(), relres_host);
-  if (status_host) std::copy(st.begin(), st.end(), status_host);
+  const i64* const it = results.data();
+  const i64* const up = it + nb;
+  const double* const rel = reinterpret_cast<const double*>(it + 2 * nb);
+  const double* const res = reinterpret_cast<const double*>(it + 3 * nb);
+  const int* const st = reinterpret_cast<const int*>(it + 4 * nb);
+  if (iters_host) std::copy(it, it + nb, iters_host);
+  if (relres_host) std::copy(rel, rel + nb, relres_host);
+  if (status_host) std::copy(st, st + nb, status_host);
   int worst = FCU_OK;
   i64 max_it = 0, sum_it = 0, sum_up = 0;
   double max_rel = 0.0, max_res = 0.0;

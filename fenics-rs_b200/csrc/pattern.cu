@@ -20,18 +20,22 @@
 namespace {
 
 __global__ void k_validity_tet(const double* __restrict__ X, const int* __restrict__ cells, i64 nc,
-                               unsigned char* __restrict__ valid) {
+                               unsigned char* __restrict__ valid, unsigned long long* __restrict__ bad) {
   for (i64 c = blockIdx.x * (i64)blockDim.x + threadIdx.x; c < nc; c += (i64)gridDim.x * blockDim.x) {
     int v[4] = {cells[4 * c], cells[4 * c + 1], cells[4 * c + 2], cells[4 * c + 3]};
-    valid[c] = tet_geometry(X, v).ok ? 1 : 0;
+    const bool ok = tet_geometry(X, v).ok;
+    valid[c] = ok ? 1 : 0;
+    if (!ok) atomicAdd(bad, 1ull);
   }
 }
 
 __global__ void k_validity_tri(const double* __restrict__ X, const int* __restrict__ cells, i64 nc,
-                               unsigned char* __restrict__ valid) {
+                               unsigned char* __restrict__ valid, unsigned long long* __restrict__ bad) {
   for (i64 c = blockIdx.x * (i64)blockDim.x + threadIdx.x; c < nc; c += (i64)gridDim.x * blockDim.x) {
     int v[3] = {cells[3 * c], cells[3 * c + 1], cells[3 * c + 2]};
-    valid[c] = tri_geometry(X, v).ok ? 1 : 0;
+    const bool ok = tri_geometry(X, v).ok;
+    valid[c] = ok ? 1 : 0;
+    if (!ok) atomicAdd(bad, 1ull);
   }
 }
 
@@ -127,6 +131,7 @@ __global__ void k_pattern_fill(const unsigned long long* __restrict__ keys, cons
                                unsigned long long sentinel, int* __restrict__ col_idx, int* __restrict__ row_ptr,
                                int* __restrict__ slot_first, unsigned* __restrict__ cnt32,
                                int* __restrict__ diag_pos, int* __restrict__ real) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) row_ptr[nn] = slot_incl[nE - 1];
   for (i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x; t < nE; t += (i64)gridDim.x * blockDim.x) {
     unsigned long long key = keys[t];
     if (key == sentinel) { real[t] = 0; continue; }
@@ -317,6 +322,26 @@ __global__ void k_contrib_permute(const int* __restrict__ order, const int* __re
   }
 }
 
+// Longest row, most contributions of a row, rows without contributions.
+__global__ void k_pattern_stats(const int* __restrict__ row_ptr, const int* __restrict__ contrib_ptr, i64 nn,
+                                int* __restrict__ out) {
+  int mr = 0, mc = 0, none = 0;
+  for (i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x; i < nn; i += (i64)gridDim.x * blockDim.x) {
+    mr = max(mr, row_ptr[i + 1] - row_ptr[i]);
+    const int c = contrib_ptr[i + 1] - contrib_ptr[i];
+    mc = max(mc, c);
+    none += c == 0;
+  }
+  mr = __reduce_max_sync(0xffffffffu, mr);
+  mc = __reduce_max_sync(0xffffffffu, mc);
+  none = __reduce_add_sync(0xffffffffu, none);
+  if ((threadIdx.x & 31) == 0) {
+    if (mr) atomicMax(&out[0], mr);
+    if (mc) atomicMax(&out[1], mc);
+    if (none) atomicAdd(&out[2], none);
+  }
+}
+
 __global__ void k_u32_to_u16(const unsigned* __restrict__ a, i64 n, unsigned short* __restrict__ b,
                              int* __restrict__ overflow) {
   for (i64 t = blockIdx.x * (i64)blockDim.x + threadIdx.x; t < n; t += (i64)gridDim.x * blockDim.x) {
@@ -355,15 +380,16 @@ void build_mesh_validity(fcu_mesh m) {
   m->valid.alloc(m->nc);
   if (m->nc == 0) { m->n_degenerate = 0; return; }
   unsigned g = grid_for(m->nc, 256, 148 * 16);
-  if (m->dim == 3) k_validity_tet<<<g, 256, 0, ctx->stream>>>(m->coords.p, m->cells.p, m->nc, m->valid.p);
-  else k_validity_tri<<<g, 256, 0, ctx->stream>>>(m->coords.p, m->cells.p, m->nc, m->valid.p);
+  DBuf<unsigned long long> count;
+  count.alloc(1);
+  CUDA_CHECK(cudaMemsetAsync(count.p, 0, count.bytes(), ctx->stream));
+  if (m->dim == 3) k_validity_tet<<<g, 256, 0, ctx->stream>>>(m->coords.p, m->cells.p, m->nc, m->valid.p, count.p);
+  else k_validity_tri<<<g, 256, 0, ctx->stream>>>(m->coords.p, m->cells.p, m->nc, m->valid.p, count.p);
   LAUNCH_CHECK(ctx);
-  std::vector<unsigned char> hv(m->nc);
-  CUDA_CHECK(cudaMemcpyAsync(hv.data(), m->valid.p, m->nc, cudaMemcpyDeviceToHost, ctx->stream));
+  unsigned long long bad = 0;
+  CUDA_CHECK(cudaMemcpyAsync(&bad, count.p, sizeof(bad), cudaMemcpyDeviceToHost, ctx->stream));
   CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
-  i64 bad = 0;
-  for (unsigned char v : hv) bad += (v == 0);
-  m->n_degenerate = bad;
+  m->n_degenerate = (i64)bad;
 }
 
 template <class T>
@@ -486,15 +512,9 @@ void build_space_pattern(fcu_space s) {
                                                                   sentinel, s->col_idx.p, s->row_ptr.p, slot_first.p,
                                                                   cnt32.p, s->diag_pos.p, real.p);
   LAUNCH_CHECK(ctx);
-  CUDA_CHECK(cudaMemcpyAsync(s->row_ptr.p + nn, &s->nnzb, sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
-  {
-    int nnzb32 = (int)nnzb;
-    CUDA_CHECK(cudaMemcpyAsync(s->row_ptr.p + nn, &nnzb32, sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
-    CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
-  }
-  DBuf<int> overflow;
-  overflow.alloc(1);
-  CUDA_CHECK(cudaMemsetAsync(overflow.p, 0, sizeof(int), ctx->stream));
+  DBuf<int> overflow;  // [a count does not fit, longest row, most contributions, rows without any]
+  overflow.alloc(4);
+  CUDA_CHECK(cudaMemsetAsync(overflow.p, 0, overflow.bytes(), ctx->stream));
   s->slot_cnt.alloc(nnzb);
   k_u32_to_u16<<<grid_for(nnzb, 256, cap), 256, 0, ctx->stream>>>(cnt32.p, nnzb, s->slot_cnt.p, overflow.p);
   LAUNCH_CHECK(ctx);
@@ -518,8 +538,17 @@ void build_space_pattern(fcu_space s) {
                                                                   s->contrib_ptr.p, s->contrib.p, s->slot_ent.p,
                                                                   overflow.p);
   LAUNCH_CHECK(ctx);
-  if (read_scalar(ctx, overflow.p))
+  k_pattern_stats<<<grid_for(nn, 256, cap), 256, 0, ctx->stream>>>(s->row_ptr.p, s->contrib_ptr.p, nn, overflow.p + 1);
+  LAUNCH_CHECK(ctx);
+  int stats[4];
+  CUDA_CHECK(cudaMemcpyAsync(stats, overflow.p, sizeof(stats), cudaMemcpyDeviceToHost, ctx->stream));
+  CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
+  if (stats[0])
     fail(FCU_ERR_UNSUPPORTED, "a node has more than 4095 incident cells or a slot more than 65535 contributions");
+  const int mr = stats[1];
+  s->max_row = mr;
+  s->max_contrib = stats[2];
+  s->nnz_ref = (nnzb - stats[3]) * (i64)s->bs * s->bs;
 
   // --- upper off-diagonal block lists (vector P1 stiffness) -------------------
   if (s->kind == FCU_SPACE_P1_VEC3) {
@@ -571,23 +600,6 @@ void build_space_pattern(fcu_space s) {
     LAUNCH_CHECK(ctx);
     CUDA_CHECK(cudaStreamSynchronize(ctx->stream));  // noff32 is a host temporary
   }
-
-  // --- host-side statistics -----------------------------------------------
-  std::vector<int> rp(nn + 1), cp(nn + 1);
-  CUDA_CHECK(cudaMemcpyAsync(rp.data(), s->row_ptr.p, (nn + 1) * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  CUDA_CHECK(cudaMemcpyAsync(cp.data(), s->contrib_ptr.p, (nn + 1) * sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  CUDA_CHECK(cudaStreamSynchronize(ctx->stream));
-  int mr = 0, mc = 0;
-  i64 empty_rows = 0;
-  for (i64 i = 0; i < nn; ++i) {
-    mr = std::max(mr, rp[i + 1] - rp[i]);
-    int cc = cp[i + 1] - cp[i];
-    mc = std::max(mc, cc);
-    empty_rows += (cc == 0);
-  }
-  s->max_row = mr;
-  s->max_contrib = mc;
-  s->nnz_ref = (nnzb - empty_rows) * (i64)s->bs * s->bs;
 
   // --- per-contribution slot map (P2 stiffness) --------------------------------
   if ((s->kind == FCU_SPACE_P2 || s->kind == FCU_SPACE_P2_NODES) && mr <= 255 && ncontrib > 0) {
