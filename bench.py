@@ -373,12 +373,12 @@ def run_cuda(args, cfg):
     traffic = _profile_traffic("spmv_bsr3_fp32_elasticity_c2.txt")
     traffic64 = _profile_traffic("spmv_bsr3_fp64_elasticity_c2.txt")
     # dominant kernel: the mixed solve's persistent loop (the whole iteration:
-    # FP32 SpMV, vector update, grid barriers), one launch of exactly 300
+    # FP32 SpMV, vector update, grid-wide exchanges), one launch of exactly 300
     # iterations after an L2 read sweep, as the profiling case pcg_c2 runs it
     pcg_iters = 300
     pcg_ms, pcg_bytes = M.time_pcg(fcu.FCU_MIXED, iterations=pcg_iters, reps=5)
     achieved = pcg_bytes / (pcg_ms * 1e-3) / 1e9
-    traffic_pcg = _profile_traffic("pcg_persistent_fp32_elasticity_c2.txt")
+    traffic_pcg = _profile_traffic("pcg_loop_fp32_elasticity_c2.txt")
 
     # e2e through the public API from pinned host buffers, every timed step
     e2e_ms = []
@@ -425,8 +425,8 @@ def run_cuda(args, cfg):
                       "gbs_cold": spmv64_bytes / (spmv64_ms * 1e-3) / 1e9, "bytes": spmv64_bytes,
                       "frac_cold": spmv64_bytes / (spmv64_ms * 1e-3) / 1e9 / peak,
                       "frac_warm": spmv64_bytes / (spmv64_warm_ms * 1e-3) / 1e9 / peak, "traffic": traffic64},
-        "roofline": {"kernel": "k_pcg_persistent<1,float,64> (the mixed PCG loop: FP32 3x3-block SpMV from "
-                               "bulk-copy staged tiles, vector update, grid barriers; one cooperative launch)",
+        "roofline": {"kernel": "k_pcg_loop<3,8,1,0,float> (the mixed PCG loop: FP32 3x3-block SpMV from bulk-copy "
+                               "staged tiles, vector update, grid-wide exchanges; one cooperative launch)",
                      "bound": "hbm", "achieved": achieved, "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
                      "frac": achieved / peak, "traffic": traffic_pcg, "bytes_per_launch": pcg_bytes,
                      "iterations_per_launch": pcg_iters, "ms_per_launch": pcg_ms,
@@ -712,7 +712,7 @@ def run_workloads(ctx, stream, peak):
     M.apply_dirichlet(b, bd, np.zeros(len(bd)))
     c5 = {"workload": "256 independent 2D P1 Poisson problems, instance i on an N_i x N_i right-diagonal unit "
                       "square, N_i ~ U{32..256} (seed 2024), kappa = exp(N(0,1)) per cell, nodal f ~ U[-1,1], "
-                      "u = 0 on each boundary, one persistent graph-captured launch, PCG to 1e-8 per instance",
+                      "u = 0 on each boundary, one launch per cluster size side by side, PCG to 1e-8 per instance",
           "instances": 256, "ndofs": V.ndofs, "nnz": M.nnz}
     for name, prec in (("mixed", fcu.FCU_MIXED), ("fp64", fcu.FCU_FP64)):
         M.batch_pcg(offs, b, tol=1e-8, max_iter=100000, precision=prec)  # tunes, captures the graph
@@ -877,9 +877,7 @@ def profile_case(name):
       transient_1024   3 Crank-Nicolson steps of the 1024^2 heat problem,
                        12 PCG iterations each
       batch_c5         the C5 batch of 256 Poisson problems, mixed PCG capped
-                       at 60 iterations per instance, 3 launches of the
-                       persistent batch kernel (shape fixed by FCU_BATCH_* if
-                       set, else tuned first)
+                       at 60 iterations per instance, solved 3 times
       p2_cube40        P2 stiffness on the unit cube 40^3 x 6 tets (384,000
                        cells, 531,441 dofs), random kappa, assembled 3 times
                        (the C3 kernel on a quarter of its cells)

@@ -658,8 +658,8 @@ class Matrix:
 
     def batch_pcg(self, offsets, b, x=None, tol=1e-8, max_iter=10000, precision=FCU_MIXED, raise_on_error=True):
         """Batched Jacobi-PCG over the diagonal blocks [offsets[i], offsets[i+1])
-        of this matrix, each solved from zero to its own tolerance in one
-        persistent launch. Returns (x, iterations, rel_residual, status, SolveInfo)."""
+        of this matrix, each solved from zero to its own tolerance by a
+        thread-block cluster. Returns (x, iterations, rel_residual, status, SolveInfo)."""
         offs = np.ascontiguousarray(offsets, dtype=np.int64)
         nb = len(offs) - 1
         x = np.empty(self.n) if x is None else x
