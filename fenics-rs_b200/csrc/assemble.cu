@@ -324,8 +324,10 @@ __global__ void __launch_bounds__(P2W * 32) k_assemble_p2_rows(
         __syncwarp();
       }
     };
-    // rows of vertices have at most two terms per entry
-    if (__all_sync(FULL, nct == 0 || (chunk & 15) < 4)) sweep(std::integral_constant<int, 2>());
+    // rows of vertices have at most two terms per entry (contributions come in
+    // order of the local index: the last one tells)
+    const int last = nct > 0 ? contrib_a[cs + nct - 1] & 15 : 0;
+    if (__all_sync(FULL, last < 4)) sweep(std::integral_constant<int, 2>());
     else sweep(std::integral_constant<int, 4>());
     const i64 rend = r0 + 3 < nrows ? r0 + 3 : nrows;
     const int base = row_ptr[r0];

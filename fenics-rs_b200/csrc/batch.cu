@@ -1032,7 +1032,7 @@ void plan_resident(fcu_matrix m, BatchWorkspace* w, const std::vector<int>& by_c
       int c = cl[i];
       while (c < cmax && active[c + 1] == active[cl[i]]) ++c;
       fit(i, c, true);
-    } else {
+    } else if (cmax > 0) {
       fit(i, cmax, false);
     }
     ctas += cl[i];

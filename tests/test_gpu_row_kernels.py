@@ -66,6 +66,33 @@ def test_p2_stiffness_rows(fcu, ctx):
         V.close()
 
 
+def test_p2_node_that_is_a_corner_of_one_cell_and_a_midpoint_of_another(fcu, ctx):
+    """Callers number the nodes of P2_NODES spaces themselves: a row may mix
+    contributions of a corner and of a mid-edge node, here with more than ten of
+    the corner's."""
+    rng = np.random.default_rng(4)
+    m = O.unit_cube(2, 2, 2)
+    cd, _ = O.p2_dofmap(m)
+    nd = int(cd.max()) + 1
+    X = np.concatenate([m.coords, rng.random((nd - m.nv, 3))])
+    cells = np.asarray(m.cells, dtype=np.int64)
+    centre = int(np.argmax(np.bincount(cells.ravel())))
+    cd = np.array(cd)
+    away = [c for c in range(len(cells)) if centre not in cells[c]]
+    for c in away[:2]:
+        cd[c, 7] = centre
+    kappa = np.exp(rng.standard_normal(len(cells)))
+    mesh = fcu.Mesh(np.ascontiguousarray(X), cells)
+    V = fcu.FunctionSpace(ctx, mesh, fcu._abi.FCU_SPACE_P2_NODES, np.ascontiguousarray(cd, dtype=np.int64))
+    M = fcu.Matrix(ctx, V).assemble_stiffness(kappa)
+    A = M.export_csc().to_scipy().toarray()
+    B = O.assemble_p2_stiffness_3d(O.Mesh(X, cells), cd, nd, kappa).to_scipy().toarray()
+    assert A.shape == B.shape
+    assert np.max(np.abs(A - B)) <= 1e-13 * np.max(np.abs(B))
+    M.close()
+    V.close()
+
+
 def _ragged(n, mean, rng, symmetric):
     rows, cols = [], []
     for i in range(n):
