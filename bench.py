@@ -378,7 +378,7 @@ def run_cuda(args, cfg):
     pcg_iters = 300
     pcg_ms, pcg_bytes = M.time_pcg(fcu.FCU_MIXED, iterations=pcg_iters, reps=5)
     achieved = pcg_bytes / (pcg_ms * 1e-3) / 1e9
-    traffic_pcg = _profile_traffic("pcg_loop_fp32_elasticity_c2.txt")
+    traffic_pcg = _profile_traffic("pcg_persistent_fp32_elasticity_c2.txt")
 
     # e2e through the public API from pinned host buffers, every timed step
     e2e_ms = []
