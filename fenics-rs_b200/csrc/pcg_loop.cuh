@@ -426,7 +426,7 @@ __device__ __forceinline__ void enter(const LoopShared<T, W>& S, int first) {
   }
 }
 
-struct Verdict {
+struct Decision {
   int done, pause, status;
   __device__ __forceinline__ bool end() const { return done || pause; }
 };
@@ -434,11 +434,11 @@ struct Verdict {
 // The decisions of decide_after_update(_mixed) on r.z and r.r, the same in
 // every thread of every CTA.
 template <bool MIXED, class T, int W>
-__device__ __forceinline__ Verdict decide(const LoopShared<T, W>& S, const double (&v)[2], bool ok, i64 iter, double rz,
+__device__ __forceinline__ Decision decide(const LoopShared<T, W>& S, const double (&v)[2], bool ok, i64 iter, double rz,
                                           double* beta) {
   const double res = sqrt(v[1]);
   const double rel = S.bnorm > 0.0 ? res / S.bnorm : res;
-  Verdict d{0, 0, 0};
+  Decision d{0, 0, 0};
   if (!ok) {
     d.done = 1;
     d.status = FCU_ERR_CUDA;
@@ -458,7 +458,7 @@ __device__ __forceinline__ Verdict decide(const LoopShared<T, W>& S, const doubl
 // after the barrier here, and read the old one last before their post of
 // r.z and r.r. True when the loop goes on.
 template <class T, int W>
-__device__ __forceinline__ bool record(LoopShared<T, W>& S, const Verdict& d, const double (&v)[2], bool ok, i64 iter,
+__device__ __forceinline__ bool record(LoopShared<T, W>& S, const Decision& d, const double (&v)[2], bool ok, i64 iter,
                                        double beta, unsigned epoch) {
   if (threadIdx.x == 32) {
     if (ok) {
@@ -607,7 +607,7 @@ __device__ __forceinline__ bool vector_phase(LoopShared<T, W>& S, double dot) {
   }
   ok = ex.wait(v2, S.ws, &S.bad);
   double beta;
-  const Verdict d = decide<MIXED>(S, v2, ok, iter, rz, &beta);
+  const Decision d = decide<MIXED>(S, v2, ok, iter, rz, &beta);
   if (!d.end()) {
     // p = z + beta p
     const T bt = (T)beta;
@@ -732,7 +732,7 @@ __device__ __forceinline__ bool vector_phase_pair(LoopShared<T, W>& S, double do
   if (i0 < np) advance(i0, r0, x0, zp0);            // read by this thread alone
   ok = ex.wait(v2, S.ws, &S.bad);
   double beta;
-  const Verdict d = decide<MIXED>(S, v2, ok, iter, rz, &beta);
+  const Decision d = decide<MIXED>(S, v2, ok, iter, rz, &beta);
   return record(S, d, v2, ok, iter, beta, ex.epoch);
 }
 
