@@ -493,6 +493,8 @@ __global__ void __launch_bounds__(RNT, 1) k_batch_resident(BatchArgs a, const in
   const unsigned ncl = cl.num_blocks(), rank = cl.block_rank();
   int parity = 0;
   const int tid = threadIdx.x;
+  // The first sum stores into the other CTAs' shared memory: all of them have to have started.
+  if (ncl > 1) cl.sync();
   // instances: as many as clusters at once, the others as clusters come free
   for (int at = (int)(blockIdx.x / ncl); at < count;) {
     const int inst = list[at];
