@@ -702,11 +702,11 @@ __global__ void __launch_bounds__(RNT, 1) k_batch_resident(BatchArgs a, const in
       a.status[inst] = status;
     }
     if ((int)(gridDim.x / ncl) >= count) break;
-    if (rank == 0 && tid < (int)ncl) {
+    if (rank == 0 && tid < 32) {  // the whole first warp, so that the mask holds lane 0
       int v = 0;
       if (tid == 0) v = (int)(gridDim.x / ncl) + atomicAdd(next, 1);
-      v = __shfl_sync(__activemask(), v, 0);
-      *cl.map_shared_rank(&turn, tid) = v;
+      v = __shfl_sync(BFULL, v, 0);
+      if (tid < (int)ncl) *cl.map_shared_rank(&turn, tid) = v;
     }
     cl.sync();
     at = turn;

@@ -29,3 +29,10 @@ def test_cluster_barrier_comes_before_the_first_remote_access():
     assert barrier < first
     assert body[:barrier].count("{") - body[:barrier].count("}") == 1
     assert barrier < body.index("for (")
+
+
+def test_the_next_instance_is_broadcast_under_a_whole_warps_mask():
+    body = _function("k_batch_resident")
+    assert "__activemask" not in body
+    ticket = body[body.index("atomicAdd(next"):]
+    assert ticket.index("__shfl_sync(BFULL, v, 0)") < ticket.index("map_shared_rank(&turn")
