@@ -1581,6 +1581,22 @@ int fitted_stages(fcu_ctx ctx, int requested, size_t stage) {
   return ns;
 }
 
+// Allows a kernel all the shared memory a CTA can have, once per device. The
+// limit belongs to the function, not to a context, and contexts launch from
+// several threads: it is never set to one launch's own need, below which
+// another thread's launch of the same kernel would be refused.
+void allow_shared_memory(const void* kern, int device, std::atomic<unsigned long long>& opted_in) {
+  const unsigned long long bit = 1ull << (device & 63);
+  if (opted_in.load() & bit) return;
+  int optin = 0;
+  cudaFuncAttributes fa;
+  CUDA_CHECK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+  CUDA_CHECK(cudaFuncGetAttributes(&fa, kern));
+  CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  optin - (int)fa.sharedSizeBytes));
+  opted_in.fetch_or(bit);
+}
+
 // Tiled 3x3-block SpMV launch: shared memory for the ring sized by the
 // longest block row; grid = resident CTAs (persistent), at most one per tile.
 template <int DIFF, class T, int TR, int BS = 3>
@@ -1594,13 +1610,8 @@ int launch_spmv_tiled_tr(fcu_matrix m, Workspace* w, const T* val, const T* p, T
   const int nstage = fitted_stages(ctx, w->stages[sizeof(T) == 4 ? 1 : 0], stage);
   const size_t smem = nstage * stage;
   auto kern = k_spmv_tiled<DIFF, T, TR, BS>;
-  static int configured_dev = -1;
-  static size_t configured_smem = 0;
-  if (configured_dev != ctx->device || configured_smem < smem) {
-    CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured_dev = ctx->device;
-    configured_smem = smem;
-  }
+  static std::atomic<unsigned long long> opted_in{0};
+  allow_shared_memory((const void*)kern, ctx->device, opted_in);
   int per_sm = 0;
   CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, SPMV_THREADS, smem));
   if (per_sm < 1) fail(FCU_ERR_UNSUPPORTED, "rows too long for the tiled SpMV");
@@ -1892,7 +1903,8 @@ void launch_loop(fcu_matrix m, Workspace* w, const LoopPlan& P, const T* val, T*
   a.ex = w->ex.p;
   auto kern = k_pcg_loop<BS, LPR, DIFF, PAIR, T>;
   const size_t smem = (size_t)P.nstage * P.stage;
-  CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  static std::atomic<unsigned long long> opted_in{0};
+  allow_shared_memory((const void*)kern, ctx->device, opted_in);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ctx->num_sms);
   cfg.blockDim = dim3(32 * (LoopShape<BS, PAIR, T>::W + 1));
