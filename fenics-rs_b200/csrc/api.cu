@@ -578,6 +578,7 @@ int fcu_mesh_create(fcu_ctx ctx, int dim, int64_t nv, const double* coords, int6
       LAUNCH_CHECK(ctx);
       if (read1(ctx, bad.p)) fail(FCU_ERR_BAD_ARG, "cell vertex index out of range");
     }
+    build_cell_det(m.get());
     build_mesh_validity(m.get());
     ctx->refs++;
     *out = m.release();

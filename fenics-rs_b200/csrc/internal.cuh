@@ -128,7 +128,7 @@ struct fcu_mesh_s {
   DBuf<double> coords;    // nv*dim, AoS as the reference stores Vec<[f64;DIM]>
   DBuf<int> cells;        // nc*nodes, int32
   DBuf<unsigned char> valid;  // 1 if |det J| >= 1e-14
-  DBuf<double> cell_det;  // nc: |det J| (built by the first load vector)
+  DBuf<double> cell_det;  // nc: |det J| (load vectors)
   i64 n_degenerate = -1;
 };
 
@@ -383,6 +383,7 @@ __device__ __forceinline__ Geo2 tri_geometry(const double* __restrict__ X, const
 }
 
 // Kernels implemented in the .cu files and used across them.
-void build_mesh_validity(fcu_mesh m);
+void build_mesh_validity(fcu_mesh m);  // waits for the stream
+void build_cell_det(fcu_mesh m);
 void build_space_pattern(fcu_space s);
 void build_transpose_positions(fcu_space s);

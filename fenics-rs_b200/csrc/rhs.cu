@@ -70,9 +70,11 @@ __global__ void k_quad_points(const double* __restrict__ X, const int* __restric
   }
 }
 
-// |det J| of every cell, computed on a mesh's first load vector and kept with
-// it (8 bytes a cell; the geometry does not change): a P2 load would otherwise
-// form it ten times per cell, once for each of its dofs.
+// |det J| of every cell, kept with the mesh (8 bytes a cell; the geometry does
+// not change): a P2 load would otherwise form it ten times per cell, once for
+// each of its dofs. Computed when the mesh is created, before that call waits
+// for its stream: spaces of any context may then read it. (Here rather than in
+// the validity pass, for this file is compiled without contraction.)
 template <int DIM>
 __global__ void k_cell_det(const double* __restrict__ X, const int* __restrict__ cells, i64 nc,
                            double* __restrict__ det) {
@@ -399,16 +401,14 @@ void quadrature_points_impl(fcu_space s, double* out_dev) {
   LAUNCH_CHECK(ctx);
 }
 
-static const double* cell_det(fcu_mesh m) {
+void build_cell_det(fcu_mesh m) {
   fcu_ctx ctx = m->ctx;
-  if (!m->cell_det.p && m->nc) {
-    m->cell_det.alloc(m->nc);
-    const unsigned g = grid_for(m->nc, 128, ctx->num_sms * 16);
-    if (m->dim == 3) k_cell_det<3><<<g, 128, 0, ctx->stream>>>(m->coords.p, m->cells.p, m->nc, m->cell_det.p);
-    else k_cell_det<2><<<g, 128, 0, ctx->stream>>>(m->coords.p, m->cells.p, m->nc, m->cell_det.p);
-    LAUNCH_CHECK(ctx);
-  }
-  return m->cell_det.p;
+  m->cell_det.alloc(m->nc);
+  if (m->nc == 0) return;
+  const unsigned g = grid_for(m->nc, 128, ctx->num_sms * 16);
+  if (m->dim == 3) k_cell_det<3><<<g, 128, 0, ctx->stream>>>(m->coords.p, m->cells.p, m->nc, m->cell_det.p);
+  else k_cell_det<2><<<g, 128, 0, ctx->stream>>>(m->coords.p, m->cells.p, m->nc, m->cell_det.p);
+  LAUNCH_CHECK(ctx);
 }
 
 template <int DIM, int K>
@@ -417,7 +417,7 @@ static void rhs_space(fcu_space s, int kind, const double* fq_dev, double p0, do
   fcu_ctx ctx = s->ctx;
   fcu_mesh m = s->mesh;
   constexpr int NQ = DIM == 2 ? 3 : 4;
-  const double* det = cell_det(m);
+  const double* det = m->cell_det.p;
   const unsigned g = grid_for(s->nnodes, 256, ctx->num_sms * 16);
   if (kind == FCU_SRC_CONSTANT) {
     k_rhs_gather<DIM, K, true><<<g, 256, 0, ctx->stream>>>(s->contrib_ptr.p, s->contrib.p, det, nullptr, p0,
@@ -446,7 +446,7 @@ void rhs_impl(fcu_space s, int kind, const double* fq_dev, double p0, double p1,
 void body_force_impl(fcu_space s, const double* f, double* b_dev) {
   fcu_ctx ctx = s->ctx;
   fcu_mesh m = s->mesh;
-  const double* det = cell_det(m);
+  const double* det = m->cell_det.p;
   k_body_force<<<grid_for(m->nv, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(
       s->contrib_ptr.p, s->contrib.p, det, f[0], f[1], f[2], m->nv, b_dev);
   LAUNCH_CHECK(ctx);
