@@ -24,9 +24,10 @@ void quadrature_points_impl(fcu_space s, double* out_dev);
 void rhs_impl(fcu_space s, int kind, const double* fq_dev, double p0, double p1, const double* nodal_dev, double* b_dev);
 void body_force_impl(fcu_space s, const double* f, double* b_dev);
 void traction_impl(fcu_space s, i64 nf, const i64* facets_dev, const double* tq_dev, double* b_dev);
-i64 boundary_facets_find(fcu_mesh m, DBuf<unsigned>& ids);
-void boundary_facets_emit(fcu_mesh m, const DBuf<unsigned>& ids, i64 nf, i64* verts_dev, i64* cell_dev, i64* local_dev);
-i64 boundary_dofs_impl(fcu_mesh m, fcu_space s_or_null, DBuf<i64>& result);
+i64 boundary_facets_find(fcu_ctx ctx, fcu_mesh m, DBuf<unsigned>& ids);
+void boundary_facets_emit(fcu_ctx ctx, fcu_mesh m, const DBuf<unsigned>& ids, i64 nf, i64* verts_dev, i64* cell_dev,
+                          i64* local_dev);
+i64 boundary_dofs_impl(fcu_ctx ctx, fcu_mesh m, fcu_space s_or_null, DBuf<i64>& result);
 int run_pcg(fcu_matrix m, const double* b_dev, const double* x0_dev, double* x_dev, double tol, i64 max_iter,
             int precision, bool gpu_semantics, const double* inv_diag_dev, fcu_solve_info* info);
 void spmv_impl(fcu_matrix m, const double* x_dev, double* y_dev);
@@ -598,7 +599,7 @@ int fcu_boundary_dofs(fcu_ctx ctx, fcu_mesh mesh, int64_t* out, int64_t* count) 
   return guarded(ctx, [&] {
     if (!mesh || !count) fail(FCU_ERR_BAD_ARG, "null argument");
     DBuf<i64> res;
-    i64 k = boundary_dofs_impl(mesh, nullptr, res);
+    i64 k = boundary_dofs_impl(ctx, mesh, nullptr, res);
     if (out) {
       if (*count < k && *count != 0) fail(FCU_ERR_BAD_ARG, "output buffer too small");
       download(ctx, out, res.p, (size_t)k);
@@ -612,10 +613,10 @@ int fcu_boundary_facets(fcu_ctx ctx, fcu_mesh mesh, int64_t* verts, int64_t* cel
   return guarded(ctx, [&] {
     if (!mesh || !count) fail(FCU_ERR_BAD_ARG, "null argument");
     DBuf<unsigned> ids;
-    const i64 nf = boundary_facets_find(mesh, ids);
+    const i64 nf = boundary_facets_find(ctx, mesh, ids);
     if (verts || cell || local) {
       DevOut<i64> V(verts, nf * mesh->dim), Cc(cell, nf), L(local, nf);
-      boundary_facets_emit(mesh, ids, nf, V.p, Cc.p, L.p);
+      boundary_facets_emit(ctx, mesh, ids, nf, V.p, Cc.p, L.p);
       V.finish(ctx);
       Cc.finish(ctx);
       L.finish(ctx);
@@ -718,7 +719,7 @@ int fcu_space_boundary_dofs(fcu_ctx ctx, fcu_space s, int64_t* out, int64_t* cou
     reject_node_space(s);
     if (!s || !count) fail(FCU_ERR_BAD_ARG, "null argument");
     DBuf<i64> res;
-    i64 k = boundary_dofs_impl(s->mesh, s, res);
+    i64 k = boundary_dofs_impl(ctx, s->mesh, s, res);
     if (out) download(ctx, out, res.p, (size_t)k);
     *count = k;
     sync(ctx);

@@ -475,9 +475,10 @@ void traction_impl(fcu_space s, i64 nf, const i64* facets_dev, const double* tq_
   LAUNCH_CHECK(ctx);
 }
 
+// (All of it on the calling context's stream, on which its buffers are
+// allocated; mesh and space are complete when their creation returns.)
 // single[t] = 1 for every boundary facet t (cell * facets per cell + local).
-static void single_facets(fcu_mesh m, DBuf<unsigned char>& single) {
-  fcu_ctx ctx = m->ctx;
+static void single_facets(fcu_ctx ctx, fcu_mesh m, DBuf<unsigned char>& single) {
   const int cap = ctx->num_sms * 16;
   const i64 n = m->nc * (m->dim + 1);
   if (m->dim == 3 && (double)m->nv * m->nv * m->nv >= 1.8e19)
@@ -508,12 +509,11 @@ static i64 flagged(fcu_ctx ctx, const unsigned char* flags, i64 n, I* out) {
 }
 
 // Boundary facets in ascending order of their sorted vertices; returns their number.
-i64 boundary_facets_find(fcu_mesh m, DBuf<unsigned>& ids) {
-  fcu_ctx ctx = m->ctx;
+i64 boundary_facets_find(fcu_ctx ctx, fcu_mesh m, DBuf<unsigned>& ids) {
   const i64 n = m->nc * (m->dim + 1);
   if (n == 0) return 0;
   DBuf<unsigned char> single;
-  single_facets(m, single);
+  single_facets(ctx, m, single);
   DBuf<unsigned> found;
   found.alloc(n);
   const i64 nf = flagged(ctx, single.p, n, found.p);
@@ -533,21 +533,20 @@ i64 boundary_facets_find(fcu_mesh m, DBuf<unsigned>& ids) {
 }
 
 // Writes the outputs (device pointers) that are not null.
-void boundary_facets_emit(fcu_mesh m, const DBuf<unsigned>& ids, i64 nf, i64* verts_dev, i64* cell_dev,
+void boundary_facets_emit(fcu_ctx ctx, fcu_mesh m, const DBuf<unsigned>& ids, i64 nf, i64* verts_dev, i64* cell_dev,
                           i64* local_dev) {
   if (nf == 0) return;
-  k_facet_emit<<<grid_for(nf, 256, m->ctx->num_sms * 16), 256, 0, m->ctx->stream>>>(
+  k_facet_emit<<<grid_for(nf, 256, ctx->num_sms * 16), 256, 0, ctx->stream>>>(
       ids.p, nf, m->cells.p, m->coords.p, m->dim, verts_dev, cell_dev, local_dev);
-  LAUNCH_CHECK(m->ctx);
+  LAUNCH_CHECK(ctx);
 }
 
 // Boundary dofs: returns the count and fills `result` (device) with the sorted list.
-i64 boundary_dofs_impl(fcu_mesh m, fcu_space s_or_null, DBuf<i64>& result) {
-  fcu_ctx ctx = m->ctx;
+i64 boundary_dofs_impl(fcu_ctx ctx, fcu_mesh m, fcu_space s_or_null, DBuf<i64>& result) {
   const i64 n = m->nc * (m->dim + 1);
   if (n == 0) return 0;
   DBuf<unsigned char> single, mark;
-  single_facets(m, single);
+  single_facets(ctx, m, single);
   const bool p2 = s_or_null && s_or_null->kind == FCU_SPACE_P2;
   const i64 ne = p2 ? s_or_null->nedges : 0, nd = m->nv + ne;
   mark.alloc(nd);

@@ -47,3 +47,33 @@ def test_load_vectors_on_another_contexts_mesh(fcu):
         for k in own:
             assert np.isfinite(own[k]).all() and np.array_equal(own[k], other[k]), k
         m.release()
+
+
+def _boundary(fcu, ctx, h, nv):
+    L, n = fcu._L(), C.c_int64(nv)
+    dofs = np.empty(nv, np.int64)
+    assert L.fcu_boundary_dofs(ctx.h, h, dofs.ctypes.data, C.byref(n)) == 0
+    out = [dofs[:n.value]]
+    V = _space(fcu, ctx, h, fcu.FCU_SPACE_P2)
+    assert L.fcu_space_boundary_dofs(ctx.h, V, None, C.byref(n)) == 0
+    p2 = np.empty(n.value, np.int64)
+    assert L.fcu_space_boundary_dofs(ctx.h, V, p2.ctypes.data, C.byref(n)) == 0
+    L.fcu_space_destroy(V)
+    assert L.fcu_boundary_facets(ctx.h, h, None, None, None, C.byref(n)) == 0
+    fv, fc, fl = np.empty((n.value, 3), np.int64), np.empty(n.value, np.int64), np.empty(n.value, np.int64)
+    assert L.fcu_boundary_facets(ctx.h, h, fv.ctypes.data, fc.ctypes.data, fl.ctypes.data, C.byref(n)) == 0
+    return out + [p2, fv, fc, fl]
+
+
+def test_boundary_of_another_contexts_mesh(fcu):
+    m = fcu.box_beam(3.0, 1.0, 1.0, 17, 9, 11)
+    with fcu.Context(0) as a, fcu.Context(0) as b:
+        h = m.handle(a)
+        launched = a.kernel_launches
+        with torch.cuda.stream(torch.cuda.ExternalStream(a.stream)):
+            torch.cuda._sleep(200_000_000)
+        other = _boundary(fcu, b, h, m.nv)
+        assert a.kernel_launches == launched
+        for x, y in zip(_boundary(fcu, a, h, m.nv), other):
+            assert np.array_equal(x, y)
+        m.release()
