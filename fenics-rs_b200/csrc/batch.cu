@@ -1150,11 +1150,12 @@ int batch_pcg_impl(fcu_matrix m, i64 nb, const i64* offsets_host, const double* 
     if (offsets_host[i + 1] < offsets_host[i]) fail(FCU_ERR_BAD_ARG, "offsets must not decrease");
   if (max_iter < 0) fail(FCU_ERR_BAD_ARG, "max_iter must be non-negative");
 
-  const bool same =
-      m->bws && m->bws->nb == nb && std::equal(m->bws->off.begin(), m->bws->off.end(), offsets_host);
+  // (a single system, tried on every small solve, leaves the caller's batch in place)
+  BatchWorkspace*& kept = on_chip_only ? m->bws_single : m->bws;
+  const bool same = kept && kept->nb == nb && std::equal(kept->off.begin(), kept->off.end(), offsets_host);
   if (!same) {
-    delete m->bws;
-    m->bws = nullptr;
+    delete kept;
+    kept = nullptr;
     std::unique_ptr<BatchWorkspace> w(new BatchWorkspace());  // kept once it is complete
     w->nb = (int)nb;
     w->off.assign(offsets_host, offsets_host + nb + 1);
@@ -1183,9 +1184,9 @@ int batch_pcg_impl(fcu_matrix m, i64 nb, const i64* offsets_host, const double* 
     w->invd.alloc(n);
     w->counter.alloc(1);
     w->results.alloc(5 * nb);
-    m->bws = w.release();
+    kept = w.release();
   }
-  BatchWorkspace* const w = m->bws;
+  BatchWorkspace* const w = kept;
   const int k = mixed ? 1 : 0;
   if (!w->planned[k]) {
     // largest first by estimated cost: stored entries x sqrt(rows), the 2D
@@ -1311,11 +1312,12 @@ int batch_pcg_impl(fcu_matrix m, i64 nb, const i64* offsets_host, const double* 
 
 void batch_config(fcu_matrix m, int precision, int* vpr, int* threads, int* cluster) {
   const int k = precision == FCU_MIXED ? 1 : 0;
-  if (!m->bws || !m->bws->tuned[k]) {
+  const BatchWorkspace* w = m->bws && m->bws->tuned[k] ? m->bws : m->bws_single;
+  if (!w || !w->tuned[k]) {
     *vpr = *threads = *cluster = 0;
     return;
   }
-  *vpr = m->bws->cfg[k].vpr;
-  *threads = m->bws->cfg[k].threads;
-  *cluster = m->bws->cfg[k].cluster;
+  *vpr = w->cfg[k].vpr;
+  *threads = w->cfg[k].threads;
+  *cluster = w->cfg[k].cluster;
 }

@@ -227,7 +227,8 @@ struct fcu_matrix_s {
   int tblk_tr[2] = {-1, -1};
   int tblk_cap[2] = {0, 0};
   Workspace* ws = nullptr;
-  BatchWorkspace* bws = nullptr;
+  BatchWorkspace* bws = nullptr;         // of the caller's batch
+  BatchWorkspace* bws_single = nullptr;  // of the whole matrix as one system (small solves)
   ~fcu_matrix_s();
 };
 

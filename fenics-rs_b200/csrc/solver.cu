@@ -1339,6 +1339,7 @@ struct Workspace {
 fcu_matrix_s::~fcu_matrix_s() {
   delete ws;
   destroy_batch_ws(bws);
+  destroy_batch_ws(bws_single);
 }
 
 namespace {

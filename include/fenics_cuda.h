@@ -250,7 +250,8 @@ int fcu_batch_pcg(fcu_ctx ctx, fcu_matrix m, int64_t nb, const int64_t* offsets,
 /* Lanes per row, threads per CTA and CTAs per instance (thread-block
  * cluster) of the batched solver for m and `precision` (all 0 before its first
  * solve): those of the queue if any instance takes it, else those of the
- * largest cluster. */
+ * largest cluster. Without a batch, those of a small system that fcu_pcg
+ * solved on chip. */
 int fcu_batch_config(fcu_matrix m, int precision, int* lanes_per_row, int* threads_per_cta,
                      int* ctas_per_cluster);
 
