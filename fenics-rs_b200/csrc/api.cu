@@ -127,6 +127,14 @@ __global__ void k_diag_pos(const int* __restrict__ rp, const int* __restrict__ c
   }
 }
 
+__global__ void k_longest_row(const int* __restrict__ rp, i64 n, int* __restrict__ out) {
+  int m = 0;
+  for (i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x)
+    m = max(m, rp[i + 1] - rp[i]);
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0) atomicMax(out, m);
+}
+
 // CSC entry k of column c -> sort key (row * n + col) for the CSR transpose.
 __global__ void k_csc_keys(const i64* __restrict__ cp, const i64* __restrict__ ri, i64 n, int* __restrict__ bad,
                            unsigned long long* __restrict__ keys, unsigned* __restrict__ idx, i64 nnz) {
@@ -433,6 +441,7 @@ fcu_matrix matrix_clone(fcu_matrix src) {
   copy(m->bdinv, src->bdinv);
   m->block_jacobi = src->block_jacobi;
   m->max_row_own = src->max_row_own;
+  m->longest_row = src->longest_row;
   m->missing_diag = src->missing_diag;
   m->has_values = src->has_values;
   if (m->space) m->space->refs++;
@@ -835,6 +844,10 @@ int fcu_matrix_from_csc(fcu_ctx ctx, int64_t n, const int64_t* colptr, const int
     k_diag_pos<<<grid_for(n, 256, cap_blocks(ctx)), 256, 0, ctx->stream>>>(m->own_row_ptr.p, m->own_col_idx.p, n,
                                                                            m->own_diag_pos.p);
     LAUNCH_CHECK(ctx);
+    CUDA_CHECK(cudaMemsetAsync(bad.p, 0, sizeof(int), ctx->stream));
+    k_longest_row<<<grid_for(n, 256, cap_blocks(ctx)), 256, 0, ctx->stream>>>(m->own_row_ptr.p, n, bad.p);
+    LAUNCH_CHECK(ctx);
+    CUDA_CHECK(cudaMemcpyAsync(&m->longest_row, bad.p, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     m->csr_of.alloc(std::max<i64>(nnz, 1));
     k_csr_of<<<grid_for(nslots, 256, cap_blocks(ctx)), 256, 0, ctx->stream>>>(src.p, nslots, m->csr_of.p);
     LAUNCH_CHECK(ctx);

@@ -216,6 +216,7 @@ struct fcu_matrix_s {
   DBuf<double> bdinv;
   bool block_jacobi = false;  // bdinv derived from the values at every solve
   int max_row_own = 0;  // longest block row of a wrapped block CSR matrix
+  int longest_row = 0;  // entries of the longest row of a wrapped CSC (0: not known)
   bool missing_diag = false;  // a wrapped block row without a diagonal block
   DBuf<int> rowblk;     // row blocks of the CSR-stream SpMV (scalar, built on first use)
   int nrowblk = 0;

@@ -1099,7 +1099,8 @@ __global__ void k_spmv_plain(const int* __restrict__ rp, const int* __restrict__
   spmv_rows<BS, VPR, false, double>(rp, ci, val, nrows, XPlain<double>{x}, em);
 }
 
-// Scalar rows of medium length (8 to 64 entries on average): VPR lanes per
+// Scalar rows of medium length (8 to 64 entries on average, none longer than
+// medium_row_limit): VPR lanes per
 // row (loop_lanes), each fetching eight entries' columns and values and then
 // their operands together, so a row of up to 8 VPR entries costs two dependent
 // round trips. No shared memory: the whole L1 serves the operand gathers.
@@ -2213,11 +2214,22 @@ void invalidate_graphs(fcu_matrix m) {
     }
 }
 
+// Longest row that k_spmv_medium takes. Its v lanes walk a row in trips of 8 v
+// entries of about 1 us each, which is hidden while the rest of the matrix takes
+// as long (the CSR-stream kernel needs some 1 us per 310,000 entries and 4 us
+// at least); the stream kernel splits such rows. Medium / stream in us, at row
+// lengths on both sides of the limit: 27-point 40^3 (1.6M entries, limit 288)
+// 226: 8.5 / 9.4, 1023: 22 / 20, 2942: 54 / 8.0; 64^3 (6.9M, 832) 527: 34 / 37,
+// 1024: 45 / 36, 19293: 465 / 61; 9-point 300^2 (0.8M, 96) 79: 4.8 / 4.8,
+// 159: 7.0 / 5.5, 2961: 91 / 6.3; 1000^2 (9M, 512) 409: 33 / 39, 709: 50 / 39.
+i64 medium_row_limit(int v, i64 nnz) { return 8 * v * (4 + nnz / 310000); }
+
 void spmv_impl(fcu_matrix m, const double* x_dev, double* y_dev) {
   fcu_ctx ctx = m->ctx;
   const double mean = m->nnodes ? (double)m->nnzb / (double)m->nnodes : 0.0;
-  if (m->bs == 1 && mean > 8.0 && mean <= 64.0) {
-    const int v = loop_lanes(mean);
+  const int longest = m->space ? m->space->max_row : m->longest_row;
+  const int v = loop_lanes(mean);
+  if (m->bs == 1 && mean > 8.0 && mean <= 64.0 && longest > 0 && longest <= medium_row_limit(v, m->nnzb)) {
     auto go = [&](auto kern) {
       launch_pdl_cfg(ctx, kern, (int)grid_for(m->nnodes * v, 256, 1 << 20), 256, 0, m->row_ptr, m->col_idx,
                      m->val64.p, m->nnodes, x_dev, y_dev);
