@@ -2533,17 +2533,14 @@ double persistent_bytes_per_iter(fcu_matrix m, bool mixed) {
   return mat + n * 3.0 * w + n * (24.0 + 3.0 * w) + n * (16.0 + 2.0 * w);
 }
 
-// Device time of one launch of the persistent loop running exactly `iters`
-// iterations (no stopping test, no residual replacement, no breakdown exit)
-// from x = 0 on b = 1, after a read sweep of `flush_bytes` that evicts L2;
-// the mean over `reps` launches, each from a fresh start.
 // Self-check of the bounded waits the persistent loop and the tiled SpMV
 // rely on, with `limit` polls each. One CTA of the tiled kernels' shape:
 // its consumer threads wait for an exchange with a second CTA that does not
-// exist and then for one among themselves alone; warp 0 waits on an mbarrier
-// nothing arrives at and then on one whose single arrival it makes. out = {first exchange passed,
-// second exchange passed, first mbarrier wait passed, second mbarrier wait
-// passed}; a correct build gives {0, 1, 0, 1}.
+// exist, then for one among themselves alone, then for two that carry a
+// reported fault; warp 0 waits on an mbarrier nothing arrives at and then on
+// one whose single arrival it makes. out = {first exchange passed, second
+// passed and neither of the faulty ones did, first mbarrier wait passed, second
+// mbarrier wait passed}; a correct build gives {0, 1, 0, 1}.
 __global__ void __launch_bounds__(SPMV_THREADS) k_wait_limits(ExchangeMem* mem, unsigned limit,
                                                               int* __restrict__ out) {
   __shared__ unsigned long long mb[2];
@@ -2569,9 +2566,21 @@ __global__ void __launch_bounds__(SPMV_THREADS) k_wait_limits(ExchangeMem* mem, 
     ex.G = 1;  // two exchanges, two arrivals
     ex.post_arrival(&failed);
     const bool b = ex.wait_arrivals(&bad, limit);
+    // an arrival that reports a fault ends this exchange, though the count is
+    // reached, and every later one, also for a CTA that has met none itself
+    bool after[2];
+    for (int k = 0; k < 2; ++k) {
+      consumer_sync<W>();
+      if (ex.ctid == 0) {
+        bad = 0;
+        failed = k == 0;
+      }
+      ex.post_arrival(&failed);
+      after[k] = ex.wait_arrivals(&bad, limit);
+    }
     if (ex.ctid == 0) {
       out[0] = a ? 1 : 0;
-      out[1] = b ? 1 : 0;
+      out[1] = b && !after[0] && !after[1] ? 1 : 0;
     }
   } else if (tid == 0) {
     out[2] = mbar_wait(&mb[0], 0, limit) ? 1 : 0;
@@ -2594,6 +2603,10 @@ void check_wait_limits_impl(fcu_ctx ctx, unsigned limit, int* results_host) {
   ctx->launches++;
 }
 
+// Device time of one launch of the persistent loop running exactly `iters`
+// iterations (no stopping test, no residual replacement, no breakdown exit)
+// from x = 0 on b = 1, after a read sweep of `flush_bytes` that evicts L2;
+// the mean over `reps` launches, each from a fresh start.
 void time_pcg_impl(fcu_matrix m, int precision, i64 iters, int reps, size_t flush_bytes, double* ms,
                    double* bytes) {
   if (m->bs != 3 || m->bdinv.p)

@@ -435,10 +435,11 @@ int fcu_time_pcg(fcu_ctx ctx, fcu_matrix m, int precision, int64_t iterations, i
                  double* ms_per_launch, double* bytes_per_launch);
 /* Self-check of the bounded waits (no reference counterpart): one CTA waits,
  * `polls` polls each (1 .. 2^20), at a grid-wide exchange of the persistent
- * PCG loop with a CTA that does not exist, then at one it completes alone, and
- * on a shared-memory mbarrier of the tiled SpMV ring that nothing arrives at,
- * then on one it arrives at itself. results[4] = {1 if the unreachable grid
- * wait passed, 1 if the reachable one passed, the same for the two mbarrier
+ * PCG loop with a CTA that does not exist, then at one it completes alone, then
+ * at two that carry a reported fault, and on a shared-memory mbarrier of the
+ * tiled SpMV ring that nothing arrives at, then on one it arrives at itself.
+ * results[4] = {1 if the unreachable grid wait passed, 1 if the reachable one
+ * passed and neither of the faulty ones did, the same for the two mbarrier
  * waits}: a correct build gives {0, 1, 0, 1}. A wait that gives up returns;
  * nothing traps, and the context stays usable. */
 int fcu_check_wait_limits(fcu_ctx ctx, uint32_t polls, int* results);
