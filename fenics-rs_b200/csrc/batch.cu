@@ -853,11 +853,11 @@ BatchArgs make_args(fcu_matrix m, BatchWorkspace* w, bool mixed, double tol, i64
   return a;
 }
 
-// Directions formed in the SpMV (FD) for FP64 and for single-instance
-// launches (the small-system path), where the saved cluster barrier pays;
-// mixed batches keep the direction phase (on the 256-problem batch the extra
-// gathers cost more than the barrier: 108.9 against 106.7 ms, while FP64 went
-// from 144.7 to 138.6 ms and single systems of 4k-16k rows gained 9-14%).
+// The streaming form makes directions in the SpMV (FD) for FP64 and for a queue
+// of one instance, where the saved cluster barrier pays; mixed queues keep the
+// direction phase. Measured with every instance streamed, as all were before
+// most moved on chip: 256 problems mixed 108.9 (FD) against 106.7 ms, FP64 138.6
+// against 144.7; single systems of 4k-16k rows gained 9-14 %.
 bool fused_direction(bool mixed, int nb) { return !mixed || nb == 1; }
 
 BatchKernel pick_kernel(bool mixed, const BatchConfig& c, int nb) {

@@ -32,8 +32,10 @@
 // 56k dofs 16.5 -> 11.2 us, 421k 47.7 -> 36.0, 1.57M 140.6 -> 118; mixed 56k
 // 11.6 -> 9.6, 421k 31.9 -> 26.6, 1.57M 87.5 -> 78.4; heat on 1.05M dofs FP64
 // 44.2 -> 33.6.
-// Every wait is bounded: one that gives up sets the fault flag, tells the
-// other CTAs through its next exchange and ends the loop.
+// Every wait is bounded. A CTA whose ring wait gives up says so in its next
+// exchange, from which all CTAs end the loop; one whose exchange gives up ends
+// it at once, and the others' next exchange gives up in turn. Either way the
+// solve's fault flag is set.
 #pragma once
 
 constexpr int MAX_RING = 16;            // stages of the loop's ring
@@ -371,8 +373,11 @@ struct FromPair {
 // Shape of the loop by block size and value type: consumer warps W, entries a
 // lane fetches in one go (E), rows a lane group takes of a tile (R).
 //  - FP64 needs the registers of 16 warps (128 a thread): with 24 or 32 warps
-//    the product spills, and a spilled operand is waited for at once. FP32
-//    fits 24 warps, which hide more of the gather latency.
+//    the product spills, and a spilled operand is waited for at once. Its plain
+//    scalar shapes spill 36 bytes even so, the others at most 8.
+//  - FP32 plain shapes run 24 warps, which hide more of the gather latency than
+//    the 72 bytes they spill (80 registers) cost: P2 system of 2.15M dofs 151 us
+//    per iteration, with 20 warps 159, with 16 174. Pairs keep 16.
 //  - 3x3 blocks: one FP64 block per lane of a 16-lane row keeps the 72-byte
 //    blocks free of bank conflicts, two rows at once hide the latency; FP32
 //    takes two blocks per lane of an 8-lane row.
@@ -480,9 +485,8 @@ __device__ __forceinline__ bool record(LoopShared<T, W>& S, const Decision& d, c
 
 // The vector half of an iteration, from this thread's share of p.Ap to the new
 // direction: both sums, alpha, beta and the decisions. Returns false when the
-// loop ends (S says how). A call of its own, so that its registers (K
-// elements of r, D^-1, p and z across the exchanges) do not add to those of
-// the product: in one body the product spilled.
+// loop ends (S says how). Inlined: the elements of r, D^-1, p and z that a
+// thread keeps across the exchanges (K pairs) are dead during the product.
 template <bool MIXED, class T, int W>
 __device__ __forceinline__ bool vector_phase(LoopShared<T, W>& S, double dot) {
   constexpr int K = 1;  // pairs of vector elements a thread keeps in registers
@@ -639,8 +643,8 @@ __device__ __forceinline__ bool vector_phase(LoopShared<T, W>& S, double dot) {
 
 // The same with the direction left to the product: z and p are kept as pairs
 // and the CTA updates the elements of its own tiles' rows, so that Ap never
-// leaves the CTA. Two exchanges per iteration instead of three, the first
-// without a fence; the price is the product's gathers of pairs.
+// leaves the CTA. Two exchanges per iteration instead of three; the price is
+// the product's gathers of pairs.
 template <bool MIXED, class T, int W>
 __device__ __forceinline__ bool vector_phase_pair(LoopShared<T, W>& S, double dot) {
   using T2 = typename Pair<T>::type;

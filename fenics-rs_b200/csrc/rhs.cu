@@ -351,7 +351,6 @@ __global__ void k_facet_emit(const unsigned* __restrict__ ids, i64 nf, const int
   }
 }
 
-// P2 boundary edges: each boundary facet adds its vertices and edge dofs.
 // Marks the dofs on the boundary facets: their vertices and, for P2, their
 // edges (ne > 0; an edge's number by bisection of the sorted edge list).
 __global__ void k_mark_boundary(const unsigned char* __restrict__ single, i64 n, const int* __restrict__ cells, int dim,

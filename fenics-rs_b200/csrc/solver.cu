@@ -39,9 +39,14 @@
 // Solves with the point-Jacobi preconditioner run instead as the persistent
 // loop of pcg_loop.cuh whenever the matrix fits it: one cooperative launch per
 // solve, one CTA per SM, bounded grid-wide exchanges in place of kernel
-// boundaries. The kernels above serve block-Jacobi solves, rows too long for
-// the loop, and FCU_PERSISTENT=0. Small scalar systems go to the batched
-// kernel as a single instance (batch.cu).
+// boundaries. Small scalar systems go to the batched kernel as a single
+// instance (batch.cu). The kernels above are left with
+//  - block-Jacobi solves (FP64: the 3x3 tiled SpMV, direction and block update);
+//  - scalar matrices with a row longer than a tile of the loop holds (about
+//    4,600 entries FP64, 6,900 FP32): CSR-stream or CSR SpMV, direction, update,
+//    and in mixed precision the replacement kernel;
+//  - FCU_PERSISTENT=0, and the SpMV timing entries, which alone reach the scalar
+//    tiled SpMV: where a row does not fit the loop it does not fit that either.
 
 #include <algorithm>
 #include <atomic>
@@ -1773,9 +1778,13 @@ int loop_lanes(double mean) { return mean <= 8.0 ? 1 : mean <= 16.0 ? 2 : mean <
 // direction and three: about what the SMs' shared memory holds. Below it an
 // exchange costs more than the pairs' wider gathers, above it less. Measured
 // (us per iteration, pairs against plain): FP64 12 MB 9.1 / 10.7, 20 MB
-// 11.2 / 11.5, 41 MB 17.9 / 18.1, 46 MB 16.1 / 15.2, 154 MB 43.2 / 36.0; mixed
-// 11 MB 9.6 / 10.8, 24 MB 12.2 / 13.3, 33 MB 17.7 / 19.0, 61 MB 22.6 / 22.4,
-// 81 MB 27.7 / 26.4.
+// 11.2 / 11.5, 41 MB 17.9 / 18.1, 46 MB 16.1 / 15.2, 55 MB 19.6 / 17.7, 154 MB
+// 43.2 / 36.0; mixed 11 MB 9.6 / 10.8, 24 MB 12.2 / 13.3, 29 MB 14.9 / 16.1. One
+// line serves both precisions and block sizes. It lies where mixed scalar rows
+// cross (39 MB 21.5 / 21.8, 40 MB 23.2 / 22.8, 50 MB 24.4 / 24.3) and a little
+// below FP64; mixed 3x3 blocks cross only at about 55 MB (37 MB 17.2 / 18.2, 44
+// MB 19.1 / 20.8, 52 MB 21.2 / 21.7, 62 MB 24.3 / 23.7) and give up to 8 %
+// between.
 constexpr double PAIR_BYTES = 36e6;
 
 // Tiles and ring of the persistent loop for m, made once per matrix and
